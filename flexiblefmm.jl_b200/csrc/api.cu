@@ -682,6 +682,9 @@ int fmmb_state_create(fmmb_plan* plan, int precision, fmmb_state** out) {
       std::lock_guard<std::mutex> lk(P.cache->mu);
       prepare_mixed_operators(*P.cache);
       prepare_mixed_levels(P);
+    } else {
+      std::lock_guard<std::mutex> lk(P.cache->mu);
+      prepare_rotations(P);
     }
     apply_tuned_state(S);                         // the launch shapes tuned for states of this kind
     FMMB_CUDA(cudaStreamSynchronize(s));

@@ -695,7 +695,7 @@ int m2l_stage(State& S) {
     m2l_mixed(S);
     return 4;
   }
-  m2l_f64(S);
+  m2l_rot(S);
   return 1;
 }
 

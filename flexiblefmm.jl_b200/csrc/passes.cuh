@@ -217,7 +217,8 @@ void gemm_expansions(int M, int K, const double* A, ColMap bm, ColMap cm, int nc
 // P2M of charges q and, when d3 (3 × N planar) is given, dipoles into M (pitch doubles per node)
 void p2m_block(State& S, const double* q, const double* d3, double* M, int64_t pitch);
 
-void m2l_f64(State& S);
+void m2l_rot(State& S);
+void prepare_rotations(Plan& P);   // the cache locked by the caller
 int p2m(State& S);          // the stages of the passes; each returns its kernel launches
 int m2m_sweep(State& S);
 int m2l_stage(State& S);

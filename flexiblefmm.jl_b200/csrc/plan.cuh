@@ -6,6 +6,7 @@
 
 #include "common.cuh"
 #include "ki.h"
+#include "m2l_rot.h"
 
 namespace fmmb {
 
@@ -26,6 +27,8 @@ struct YukawaLevel {
   std::mutex mu;
   DBuf<uint16_t> reps16;
   DBuf<float> row_scale;
+  // the FP64 M2L's translations along z of this width (built when an FP64 state first needs them)
+  DBuf<double> rot_t;
 };
 
 // OperatorCache (src/operators/cache.jl:5-83): the base width, the host operators at the base
@@ -50,6 +53,10 @@ struct Cache {
   DBuf<float> row_scale;
   DBuf<uint32_t> perm16;
   bool split_ready = false;
+  // the FP64 M2L (m2l_rot.cu): per class the rotation of its representative offset to the z axis
+  // and the translation along z (Yukawa3D: the level widths')
+  std::shared_ptr<const RotHost> rot;
+  DBuf<double> rot_d, rot_cs, rot_csf, rot_t;
   // Yukawa3D: κ, the operators per width (keyed by the exponent e of w = ldexp(W0, e); built on
   // first use and shared by every cache of the same device, order, κ and width), and the sphere
   // quadrature of the projections
@@ -127,6 +134,7 @@ struct Plan {
   std::vector<const double*> lv_reps, lv_m2m, lv_l2l;
   DBuf<uint64_t> d_lv_reps;
   DBuf<double> d_kh2;
+  DBuf<uint64_t> d_lv_rot;                // the FP64 path: per level the translations along z of the classes
   // the mixed path: per level the split class operators and their inverse row scales (the cache's
   // for the homogeneous kernels, the level width's own for Yukawa3D), built with the first mixed
   // state; the Yukawa levels they come from stay held by the plan
@@ -165,10 +173,8 @@ struct Plan {
 struct State {
   Plan* plan = nullptr;
   int precision = FMMB_PRECISION_FP64;
-  // launch shapes chosen by the tuner (tune.cu): near-field warps per CTA (4 or 8), the FP64
-  // M2L's alternative chunk width
+  // the launch shape chosen by the tuner (tune.cu): near-field warps per CTA (4 or 8)
   int near_warps = 4;
-  int f64_nb_alt = 0;
   DBuf<double> xs, ys, zs, q;             // sources and charges in tree order
   DBuf<double> f3;                        // Stokeslet states: the forces in tree order (fx, fy, fz)
   DBuf<double> sd;                        //   stresslet strengths, stressvecs, doublets (3 × N planar each)
@@ -219,7 +225,7 @@ int tuned_block_size(const Plan& P);
 void apply_tuned_state(State& S);
 // times the launch shapes on the state's inputs, keeps the fastest for its kind and applies them
 // (tune_blocks: also the plan's M2L block size, shared by the plan's other states); out: the
-// chosen block size, FP64 chunk width variant, near-field warps, and the M2L and near-field ms
+// chosen block size, 0, near-field warps, and the M2L and near-field ms
 void autotune(State& S, const double* xyz_dev, const double* tau_dev, bool tune_blocks, double* out);
 void build_target_pairs(Plan& P);
 // passes.cu

@@ -1,17 +1,16 @@
 // The autotuner of the launch shapes: tile and block shapes chosen by timing them on the
 // caller's own inputs (the reference has no tuner).
 //
-// Three shapes are free, in that no result depends on them (each target's sums are taken in the
+// Two shapes are free, in that no result depends on them (each target's sums are taken in the
 // list's order whatever the blocking, and a near-field warp owns its leaf group):
 //   - the targets per M2L block (32, 64 or 128; a plan property: its blocks are re-cut from the
 //     pairs per target), for both M2L kernels;
-//   - the FP64 M2L's chunk width (two compiled widths per expansion length);
 //   - the near-field warps per CTA (4 or 8).
 // fmmb_autotune times each candidate on the state's own inputs (CUDA events on the context's
 // stream, the median of three after one warm-up), keeps the fastest, applies it, and records it
 // for every later plan and state of the same kind: method, kernel, order, precision path and the
 // number of points rounded down to a power of two. Plans created afterwards take the recorded
-// block size; states take the recorded chunk width and warps.
+// block size; states take the recorded warps.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -23,7 +22,7 @@ namespace fmmb {
 namespace {
 
 struct Tuned {
-  int tb = 0, nb_alt = 0, near_w = 4;
+  int tb = 0, near_w = 4;
 };
 using Kind = std::tuple<int, int, int, int, int>;   // method, kernel, p, precision (-1: any), log2 N
 
@@ -76,7 +75,6 @@ void apply_tuned_state(State& S) {
   std::lock_guard<std::mutex> lk(g_mu);
   auto it = g_tuned.find(kind_of(*S.plan, S.precision));
   if (it == g_tuned.end()) return;
-  S.f64_nb_alt = it->second.nb_alt;
   S.near_warps = it->second.near_w;
 }
 
@@ -94,22 +92,17 @@ void autotune(State& S, const double* xyz, const double* tau, bool tune_blocks, 
     gather_inputs(S, xyz, tau);
     upward_pass(S);
   }
-  // the M2L: block sizes × (FP64) chunk widths
+  // the M2L's block sizes
   std::vector<int> tbs = {P.TB};
   if (tune_blocks) tbs = {32, 64, 128};
-  const bool f64 = S.precision == FMMB_PRECISION_FP64;
   double best = 1e300;
-  int best_tb = P.TB, best_alt = S.f64_nb_alt;
+  int best_tb = P.TB;
   for (int tb : tbs) {
     if (tb != P.TB) build_blocks(P, tb);
-    for (int alt = 0; alt < (f64 ? 2 : 1); ++alt) {
-      S.f64_nb_alt = f64 ? alt : S.f64_nb_alt;
-      const double ms = time_ms(s, [&] { m2l_stage(S); });
-      if (ms < best) { best = ms; best_tb = tb; best_alt = S.f64_nb_alt; }
-    }
+    const double ms = time_ms(s, [&] { m2l_stage(S); });
+    if (ms < best) { best = ms; best_tb = tb; }
   }
   if (P.TB != best_tb) build_blocks(P, best_tb);
-  S.f64_nb_alt = best_alt;
   // the near field at the sources (harmonic methods with charges: Laplace3D and Yukawa3D)
   double best_near = 0;
   int best_w = S.near_warps;
@@ -129,14 +122,13 @@ void autotune(State& S, const double* xyz, const double* tau, bool tune_blocks, 
     std::lock_guard<std::mutex> lk(g_mu);
     Tuned t;
     t.tb = best_tb;
-    t.nb_alt = best_alt;
     t.near_w = best_w;
     g_tuned[kind_of(P, S.precision)] = t;
     if (tune_blocks) g_tuned[kind_of(P, -1)] = t;
   }
   if (out) {
     out[0] = best_tb;
-    out[1] = best_alt;
+    out[1] = 0;                          // the FP64 M2L has one chunk width
     out[2] = best_w;
     out[3] = best;
     out[4] = best_near;
