@@ -81,174 +81,6 @@ __global__ void k_gather_dipoles(const double* __restrict__ xyz, const double* _
   d3[2 * n + k] = dip ? dip[3 * j + 2] : 0.0;
 }
 
-// P2M of charges and dipoles d (src/operators/harmonics.jl:708-738): one thread per (node, order
-// m); per source the charge's chain of order m, and the dipole's three terms from the chains of
-// orders m − 1, m, m + 1 of degree n′ = n − 1 (the derivative identities, with the moment in box
-// units d·s, harmonics.jl:436):
-//   chain m − 1: (n, m) += ½ cm(n, m) · (−(dx ur − dy ui), dx ui + dy ur)
-//   chain m:     (n, m) += cz(n, m) dz · (ur, −ui)
-//   chain m + 1: (n, m) += ½ cp(n, m) · (dx ur + dy ui, dy ur − dx ui)   (m = 0: cp(n, 0) (dx ur + dy ui), 0)
-template <int P>
-__global__ void k_p2m_dip(const int* __restrict__ nodes, int nn, const int4* __restrict__ cell, const int* __restrict__ plo,
-                          const int* __restrict__ phi, const double* __restrict__ xs, const double* __restrict__ ys,
-                          const double* __restrict__ zs, const double* __restrict__ q, const double* __restrict__ d3,
-                          int64_t npts, Geometry geo, const double* __restrict__ scale, int64_t pitch,
-                          double* __restrict__ M) {
-  __shared__ double s_t[5 * TRI_MAX];   // a, b, cz, cm, cp
-  __shared__ double s_e[PMAX];
-  for (int i = threadIdx.x; i < 5 * TRI_MAX; i += blockDim.x) s_t[i] = c_tab[i];
-  for (int i = threadIdx.x; i < PMAX; i += blockDim.x) s_e[i] = c_e[i];
-  __syncthreads();
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
-  const int m = g / nn, qn = g % nn;
-  if (m > P) return;
-  const int node = nodes[qn];
-  const int4 c = cell[node];
-  const Geometry gn = geo.at(node);
-  const double w = ldexp(geo.W0, -c.w), s = scale[c.w];
-  const double cx = gn.center(0, c.x, w), cy = gn.center(1, c.y, w), cz = gn.center(2, c.z, w);
-  double ar[P + 1], ai[P + 1];
-#pragma unroll
-  for (int n = 0; n <= P; ++n) { ar[n] = 0; ai[n] = 0; }
-  for (int j = plo[node]; j <= phi[node]; ++j) {
-    const double x = (xs[j] - cx) * s, y = (ys[j] - cy) * s, z = (zs[j] - cz) * s;
-    const double r2 = x * x + y * y + z * z;
-    const double tau = q[j], dx = d3[j] * s, dy = d3[npts + j] * s, dz = d3[2 * npts + j] * s;
-    // sectoral values of orders m − 1, m, m + 1
-    double sr = 1.0, si = 0.0, lr = 0, li = 0, mr = 1.0, mi = 0.0, hr = 0, hi = 0;
-    for (int k = 1; k <= m + 1; ++k) {
-      const double e = s_e[k - 1];
-      const double nr = -e * (x * sr - y * si), ni = -e * (x * si + y * sr);
-      if (k == m) { lr = sr; li = si; }
-      sr = nr; si = ni;
-      if (k == m) { mr = sr; mi = si; }
-      if (k == m + 1) { hr = sr; hi = si; }
-    }
-    if (m == 0) { mr = 1.0; mi = 0.0; }
-    // the chain of order k from its sectoral value (vr, vi), calling f(n′, ur, ui) for n′ = k..nmax
-    auto chain = [&](int k, double vr, double vi, int nmax, auto&& f) {
-      double pr = 0, pi = 0, cr = vr, ci = vi;
-#pragma unroll
-      for (int n = 0; n <= P; ++n) {
-        if (n < k || n > nmax) continue;
-        if (n > k) {
-          const int t = tri(n, k);
-          const double az = s_t[t] * z, br = s_t[TRI_MAX + t] * r2;
-          const double nr = az * cr - br * pr, ni = az * ci - br * pi;
-          pr = cr; pi = ci; cr = nr; ci = ni;
-        }
-        f(n, cr, ci);
-      }
-    };
-    chain(m, mr, mi, P, [&](int n, double ur, double ui) {
-      ar[n] += tau * ur;
-      ai[n] -= tau * ui;
-      if (n < P) {
-        const double cc = s_t[2 * TRI_MAX + tri(n + 1, m)] * dz;
-        ar[n + 1] += cc * ur;
-        ai[n + 1] -= cc * ui;
-      }
-    });
-    if (m >= 1)
-      chain(m - 1, lr, li, P - 1, [&](int n, double ur, double ui) {
-        const double cc = 0.5 * s_t[3 * TRI_MAX + tri(n + 1, m)];
-        ar[n + 1] += -cc * (dx * ur - dy * ui);
-        ai[n + 1] += cc * (dx * ui + dy * ur);
-      });
-    if (m + 1 <= P - 1)
-      chain(m + 1, hr, hi, P - 1, [&](int n, double ur, double ui) {
-        if (m >= 1) {
-          const double cc = 0.5 * s_t[4 * TRI_MAX + tri(n + 1, m)];
-          ar[n + 1] += cc * (dx * ur + dy * ui);
-          ai[n + 1] += cc * (dy * ur - dx * ui);
-        } else {
-          ar[n + 1] += s_t[4 * TRI_MAX + tri(n + 1, 0)] * (dx * ur + dy * ui);
-        }
-      });
-  }
-  double* col = M + (int64_t)node * pitch;
-#pragma unroll
-  for (int n = 0; n <= P; ++n) {
-    if (n < m) continue;
-    if (m == 0) col[n * n] = ar[n];
-    else { col[n * n + 2 * m - 1] = ar[n]; col[n * n + 2 * m] = ai[n]; }
-  }
-}
-
-// ---------------------------------------------------------------- P2M
-// one thread per (node, order m): M_n^m += τ conj Υ̃_n^m((y − c)/w) over the node's sources,
-// n = m..P, the chain of order m started from its own sectoral value (harmonics.jl:682-743)
-// Yukawa3D (YK): the degree-n terms weighted by u_n(κ̂|x̂|), κ̂² = kh2[level]
-// (harmonics_yukawa.jl:281-296). R = float on the mixed path of Laplace3D (box-centred, scaled
-// coordinates in [−½, ½]³, sums over the box's sources in FP32, written as doubles: about 2⁻²⁴
-// per coefficient, below the FP16x3 M2L's 2⁻²² that consumes them).
-template <int P, bool YK, typename R>
-__global__ void k_p2m(const int* __restrict__ nodes, int nn, const int4* __restrict__ cell, const int* __restrict__ plo,
-                      const int* __restrict__ phi, const double* __restrict__ xs, const double* __restrict__ ys,
-                      const double* __restrict__ zs, const double* __restrict__ q, Geometry geo,
-                      const double* __restrict__ scale, int64_t pitch, double* __restrict__ M,
-                      const double* __restrict__ kh2) {
-  static_assert(!YK || sizeof(R) == 8, "Yukawa3D's P2M runs in FP64");
-  // the recurrence tables in shared memory: the lanes of a warp run different orders and would
-  // serialise on the constant cache
-  __shared__ R s_ab[2 * TRI_MAX];
-  __shared__ R s_e[PMAX];
-  for (int i = threadIdx.x; i < 2 * TRI_MAX; i += blockDim.x) s_ab[i] = ctab<R>(i);
-  for (int i = threadIdx.x; i < PMAX; i += blockDim.x) s_e[i] = ce<R>(i);
-  __syncthreads();
-  // thread g: order m = g / nn of node g % nn; the lanes of a warp share the order, so the
-  // recurrence's branches on n versus m are uniform
-  int g = blockIdx.x * blockDim.x + threadIdx.x;
-  int m = g / nn, qn = g % nn;
-  if (m > P) return;
-  int node = nodes[qn];
-  int4 c = cell[node];
-  const Geometry gn = geo.at(node);
-  double w = ldexp(geo.W0, -c.w), s = scale[c.w];
-  double cx = gn.center(0, c.x, w), cy = gn.center(1, c.y, w), cz = gn.center(2, c.z, w);
-  const double k2 = YK ? kh2[c.w] : 0.0;
-  R ar[P + 1], ai[P + 1];
-#pragma unroll
-  for (int n = 0; n <= P; ++n) { ar[n] = 0; ai[n] = 0; }
-  int j1 = phi[node];
-  for (int j = plo[node]; j <= j1; ++j) {
-    const R x = R((xs[j] - cx) * s), y = R((ys[j] - cy) * s), z = R((zs[j] - cz) * s);
-    const R r2 = x * x + y * y + z * z;
-    R sr = 1, si = 0;
-    for (int k = 1; k <= m; ++k) {
-      const R e = s_e[k - 1];
-      const R nr = -e * (x * sr - y * si), ni = -e * (x * si + y * sr);
-      sr = nr; si = ni;
-    }
-    const R tau = R(q[j]);
-    double u[P + 1];
-    if constexpr (YK) yukawa_u<P>(k2 * (double)r2, u);
-    R pr = 0, pi = 0, cr = 0, ci = 0;
-#pragma unroll
-    for (int n = 0; n <= P; ++n) {
-      R tn = tau;
-      if constexpr (YK) tn = tau * u[n];
-      if (n == m) {
-        cr = sr; ci = si; pr = 0; pi = 0;
-        ar[n] += tn * cr; ai[n] -= tn * ci;
-      } else if (n > m) {
-        int t = tri(n, m);
-        const R az = s_ab[t] * z, br = s_ab[TRI_MAX + t] * r2;
-        const R nr = az * cr - br * pr, ni = az * ci - br * pi;
-        pr = cr; pi = ci; cr = nr; ci = ni;
-        ar[n] += tn * nr; ai[n] -= tn * ni;
-      }
-    }
-  }
-  double* col = M + (int64_t)node * pitch;
-#pragma unroll
-  for (int n = 0; n <= P; ++n) {
-    if (n < m) continue;
-    if (m == 0) col[n * n] = (double)ar[n];
-    else { col[n * n + 2 * m - 1] = (double)ar[n]; col[n * n + 2 * m] = (double)ai[n]; }
-  }
-}
-
 // ---------------------------------------------------------------- GEMM over mapped columns (M2M, L2L)
 
 // one FP64 tensor-core MMA, D(8×8) += A(8×4)·B(4×8): this lane holds A[g][t], B[t][g] and
@@ -477,29 +309,6 @@ __global__ void k_bounds_batch(const double* __restrict__ xyz, const int64_t* __
 }
 
 // P2M of charges q (and, when d3 is given, dipoles d3: 3 × N planar) into M (pitch per node)
-template <int P>
-void launch_p2m(State& S, const double* q, const double* d3, double* M, int64_t pitch) {
-  Plan& P_ = *S.plan;
-  int nth = P_.n_s2m * (P + 1);
-  if (nth == 0) return;
-  if (d3) {
-    k_p2m_dip<P><<<nblk(nth, 128), 128, 0, P_.ctx->stream>>>(P_.s2m_nodes.p, P_.n_s2m, P_.cell.p, P_.plo.p, P_.phi.p, S.xs.p,
-                                                           S.ys.p, S.zs.p, q, d3, P_.N, geometry(P_), P_.d_scale.p,
-                                                           pitch, M);
-    FMMB_LAUNCH_CHECK();
-    return;
-  }
-  // FP32 on the mixed path of Laplace3D (charges only), FP64 otherwise
-  auto kern = P_.cache->kernel == FMMB_KERNEL_YUKAWA3D ? k_p2m<P, true, double>
-              : (S.precision == FMMB_PRECISION_MIXED && P_.cache->kernel == FMMB_KERNEL_LAPLACE3D) ? k_p2m<P, false, float>
-                                                                                                  : k_p2m<P, false, double>;
-  kern<<<nblk(nth, 128), 128, 0, P_.ctx->stream>>>(P_.s2m_nodes.p, P_.n_s2m, P_.cell.p, P_.plo.p, P_.phi.p, S.xs.p, S.ys.p,
-                                                 S.zs.p, q, geometry(P_), P_.d_scale.p, pitch, M, P_.d_kh2.p);
-  FMMB_LAUNCH_CHECK();
-}
-
-
-
 }  // namespace
 
 // ---------------------------------------------------------------- direct sums, FP64
@@ -595,15 +404,6 @@ void gather_inputs_dipoles(State& S, const double* xyz_dev, const double* tau_de
 }
 
 
-void p2m_block(State& S, const double* q, const double* d3, double* M, int64_t pitch) {
-  switch (S.plan->cache->p) {
-#define X(pp) case pp: launch_p2m<pp>(S, q, d3, M, pitch); break;
-    FMMB_P_CASES(X)
-#undef X
-    default: throw Error(FMMB_ERR_UNSUPPORTED, "p out of range");
-  }
-}
-
 void gemm_columns(int M, int K, const double* A, ColMap bm, ColMap cm, int ncols, int LD, int NP, int accumulate,
                   int num_sms, cudaStream_t s) {
   gemm_cols(M, K, A, bm, cm, ncols, LD, NP, accumulate, num_sms, s);
@@ -617,13 +417,9 @@ void gemm_expansions(int M, int K, const double* A, ColMap bm, ColMap cm, int nc
 int p2m(State& S) {
   if (S.plan->cache->method == FMMB_METHOD_CUBE_KI) return ki_p2m(S);
   if (S.plan->cache->method == FMMB_METHOD_KI_CIRCLE) return kic_p2m(S);
-  switch (S.plan->cache->p) {
-#define X(pp) case pp: launch_p2m<pp>(S, S.q.p, S.has_dip ? S.dip.p : nullptr, S.M.p, (int64_t)S.plan->cache->ld); break;
-    FMMB_P_CASES(X)
-#undef X
-    default: throw Error(FMMB_ERR_UNSUPPORTED, "p out of range");
-  }
-  return S.plan->n_s2m > 0;
+  const double *q = S.q.p, *d3 = S.has_dip ? S.dip.p : nullptr;
+  double* M = S.M.p;
+  return p2m_blocks(S, 1, &q, &d3, &M, S.plan->cache->ld);
 }
 
 int m2m_sweep(State& S) {

@@ -213,9 +213,9 @@ void gemm_columns(int M, int K, const double* A, ColMap bm, ColMap cm, int ncols
 // M2M and L2L), without multiplying that padding
 void gemm_expansions(int M, int K, const double* A, ColMap bm, ColMap cm, int ncols, int LD, int NP, int accumulate,
                      int num_sms, cudaStream_t s);
-// P2M of the childless sourced nodes with charges q (tree order) into the block at M (node pitch)
-// P2M of charges q and, when d3 (3 × N planar) is given, dipoles into M (pitch doubles per node)
-void p2m_block(State& S, const double* q, const double* d3, double* M, int64_t pitch);
+// P2M of the childless sourced nodes (p2m.cu): nsets charge sets (tree order) and, all or none, dipoles
+// (3 × N planar) into the blocks at M[a], pitch doubles per node; returns the launches
+int p2m_blocks(State& S, int nsets, const double* const* q, const double* const* d3, double* const* M, int64_t pitch);
 
 void m2l_rot(State& S);
 void prepare_rotations(Plan& P);   // the cache locked by the caller

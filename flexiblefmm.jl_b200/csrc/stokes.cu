@@ -465,10 +465,15 @@ void stokes_build(State& S, const double* xyz_dev, const StokesDensities& d) {
                                                      dens ? S.sd.p : nullptr, S.q.p, dens ? S.dip4.p : nullptr);
     FMMB_LAUNCH_CHECK();
   }
-  // P2M, one block at a time (charges, and the dipoles of the stresslets and doublets)
-  for (int a = 0; a < 3; ++a)
-    p2m_block(S, S.f3.p + a * n, dens ? S.dip4.p + 3 * a * n : nullptr, S.M.p + (int64_t)a * LD, pitch);
-  p2m_block(S, S.q.p, dens ? S.dip4.p + 9 * n : nullptr, S.M.p + 3 * (int64_t)LD, pitch);
+  // P2M of the four blocks (charges, and the dipoles of the stresslets and doublets)
+  const double *q4[4], *d4[4];
+  double* M4[4];
+  for (int a = 0; a < 4; ++a) {
+    q4[a] = a < 3 ? S.f3.p + a * n : S.q.p;
+    d4[a] = dens ? S.dip4.p + 3 * a * n : nullptr;
+    M4[a] = S.M.p + (int64_t)a * LD;
+  }
+  p2m_blocks(S, 4, q4, d4, M4, pitch);
   // M2M, level by level: the stacked children of each block (Ψ̂ with the coupling), one product each
   for (int l = P.L - 2; l >= 2; --l) {
     const int c0 = P.level_start[l + 1], ng = P.level_groups[l + 1];
