@@ -682,7 +682,8 @@ int fmmb_state_create(fmmb_plan* plan, int precision, fmmb_state** out) {
       std::lock_guard<std::mutex> lk(P.cache->mu);
       prepare_mixed_operators(*P.cache);
       prepare_mixed_levels(P);
-    } else {
+    }
+    if (P.cache->method == FMMB_METHOD_SPHERICAL_HARMONICS) {
       std::lock_guard<std::mutex> lk(P.cache->mu);
       prepare_rotations(P);
     }

@@ -1,30 +1,34 @@
-// M2L of the plain FP64 path by rotations: one launch for all levels, a CTA of G groups of warps,
-// each group the far pairs of one block of targets (src/device_passes.jl:565-580, the class-wise
-// translation of harmonics.jl:531-645).
+// The FP64 translations of the harmonic methods by rotations: M2L of the plain path (one launch for all
+// levels), M2M and L2L of every path (a launch per level; src/device_passes.jl:565-580, the translations
+// of harmonics.jl:531-645).
 //
-// A class representative is A_c = R_cᵀ T_c R_c exactly, and so is every far offset's translation:
-// R rotates the offset to the z axis (it mixes the orders of one degree), T_c translates along z (it
-// mixes the degrees of one order). The dense product costs (p+1)⁴ multiply-adds per pair, the three
-// factors 2(p+1)³: 2,673 against 14,641 at p = 10, 9,843 against 83,521 at p = 16. R is a rotation by
-// the offset's azimuth about z, a 2 × 2 rotation of each (n, m) by mφ (with the sign (−1)^(n+m) for
-// offsets that point down), then one by the polar angle about y, which the class's offsets share.
-// Per class and chunk of NC = 32·C pairs the multipoles lie in a shared-memory tile [pair][entry],
-// a lane owns C pairs, and the warps split the degrees (orders) between them:
-//   rotate     per degree: z rotation of the column read, then y_j += d_jk x_k in registers, the
-//              class's coefficients broadcast from shared memory
-//   translate  per order over the degrees, the real and the imaginary parts with the same
-//              coefficients
+// Every translation operator is A = R⁻¹ T R exactly: R rotates the offset to the z axis (it mixes the
+// orders of one degree), T translates along z (it mixes the degrees of one order). The dense product
+// costs (p+1)⁴ multiply-adds per pair, the three factors 2(p+1)³: 2,673 against 14,641 at p = 10, 9,843
+// against 83,521 at p = 16. R is a rotation by the offset's azimuth about z, a 2 × 2 rotation of each
+// (n, m) by mφ (with the sign (−1)^(n+m) for offsets that point down), then one by the polar angle about
+// y, which the offsets of a class share (M2M and L2L: all eight children).
+// Per chunk of NC = 8·NG pairs of one class the inputs lie in a shared-memory tile [pair][entry], and the
+// warps split the degrees (orders) between them:
+//   rotate     per degree: z rotation of the inputs as they are read, then the product with the class's
+//              (l + 1) × (l + 1) coefficients
+//   translate  per order over the degrees, the real and the imaginary parts with the same coefficients
 //   rotate     back with the same coefficients: R_y(−θ) = Σ R_y(θ) Σ, Σ = diag((−1)^m) (the right Σ
-//              sits in T_c, the left one in the signs of the z rotation)
-//   scatter    into the targets' partial locals: each target's entry takes its pairs one by one in
-//              the list's order, starting from the value in memory (the block owns its targets:
-//              deterministic, no atomics, and the sums depend neither on where the chunks end nor on
-//              the other targets of the block); the warp then sends the next chunk's multipoles
-//              (cp.async) into the rows it has read
-// The products are FP64 FMAs with the pairs across the lanes: blocks of 1 to p + 1 would fill a third
-// to two thirds of the 8 × 8 × 4 tiles of the FP64 tensor cores, whose rate is the FMA units'. What
-// bounds it is shared memory: the tile is read and written three times per pair, and each
-// coefficient's broadcast serves C pairs per lane.
+//              sits in T, the left one in the signs of the z rotation)
+//   scatter    into the outputs: each target's entry takes its pairs one by one in the list's order,
+//              starting from the value in memory (a target has one owner: deterministic, no atomics, and
+//              the sums depend neither on where the chunks end nor on the other targets); the warp then
+//              sends the next chunk's inputs (cp.async) into the rows it has read
+// The products run on the FP64 tensor cores, 8 pairs × 4 inputs as A and the coefficients as B, laid out
+// in fragments on the host. What bounds the kernel is shared memory, not the FP64 rate (equal on the FMA
+// units): with a pair per lane each coefficient is a broadcast per 32 pairs and multiply-add (180
+// wavefronts a pair at p = 10, against 67 for the fragments, each of which serves NG groups), and the
+// blocks of 1 to p + 1 pad the 8 × 8 × 4 tiles by half, which costs less than it saves. Measured, M2L of a
+// uniform cloud (FMAs with a pair per lane → this): 400,000 points p = 10 5.98 → 5.42 ms, p = 14 12.5 →
+// 11.6, p = 16 19.8 → 16.5; 31,000 points on a sphere p = 16 0.66 → 0.61; p = 20 120,000 points 1.20 →
+// 1.24. The dense products before it: 9.4 ms at p = 10, 57 at p = 16. M2M and L2L (dense GEMMs → this):
+// 0.146 → 0.071 and 0.103 → 0.083 ms at 400,000 points p = 10, 0.536 → 0.157 and 0.425 → 0.161 at p = 16.
+// Loading the next step's operands ahead within a product spilled (5.4 → 7.7 ms).
 #include <algorithm>
 #include <numeric>
 
@@ -56,41 +60,47 @@ struct RotSched {
   uint8_t order[2][PMAX + 1];
 };
 
-// T_c of one class from its dense representative: T^m_{ll'} = the (Re l m, Re l' m) entry of
-// D A D⁻¹, negated for odd m on both sides' behalf (Σ above): a thread per entry
-__global__ void k_rot_translations(const double* __restrict__ reps, const double* __restrict__ dtab,
-                                   const double* __restrict__ cstab, RotLayout lay, int LD, double* __restrict__ out) {
-  const int p = lay.p, c = blockIdx.x;
-  const double* A = reps + (int64_t)c * LD * LD;
-  const double* d = dtab + (int64_t)c * lay.nd;
+// the translation a launch performs: between far boxes, of the children's multipoles to their parent,
+// of the parent's local to its children
+enum : int { ROT_M2L = 0, ROT_M2M = 1, ROT_L2L = 2 };
+
+// T of class c0 + blockIdx.x from its dense operator A (column-major, lda; stride per class):
+// T^m_{ll'} = the (Re l m, Re l' m) entry of D A D⁻¹, negated for odd m on both sides' behalf (Σ
+// above): a thread per entry. Multipoles transform by the conjugate of the locals' rotation.
+__global__ void k_rot_translations(const double* __restrict__ dense, int lda, int64_t stride, int mode, int c0,
+                                   const double* __restrict__ dtab, const double* __restrict__ cstab, RotLayout lay,
+                                   double* __restrict__ out) {
+  const int p = lay.p, c = c0 + blockIdx.x;
+  const double* A = dense + blockIdx.x * stride;
+  const double sin_in = mode == ROT_L2L ? 1.0 : -1.0, sin_out = mode == ROT_M2M ? -1.0 : 1.0;
+  const double* d = dtab + (int64_t)c * 32 * lay.nd;
   const double* cs = cstab + (int64_t)c * 2 * (p + 1);
-  double* T = out + (int64_t)c * lay.nt;
-  for (int i = threadIdx.x; i < lay.nt; i += blockDim.x) T[i] = 0.0;
+  double* T = out + (int64_t)blockIdx.x * 32 * lay.nt;
+  for (int i = threadIdx.x; i < 32 * lay.nt; i += blockDim.x) T[i] = 0.0;
   __syncthreads();
   const int np = (p + 1) * (p + 1) * (p + 1);
   for (int i = threadIdx.x; i < np; i += blockDim.x) {
     const int m = i % (p + 1), l = i / (p + 1) % (p + 1), l2 = i / ((p + 1) * (p + 1));
     if (m > l || m > l2) continue;
-        double sum = 0;
+    double sum = 0;
     for (int b = 0; b <= l2; ++b) {
       // the column of D⁻¹ = Z⁻¹ Σ d Σ: order b of degree l2 from (l2, m)
-      const double v = d[lay.re_col(l2, m) + b] * ((m + b) & 1 ? -1.0 : 1.0);
-      const double vr = cs[2 * b] * v, vi = -cs[2 * b + 1] * v;
-      const double* Ar = A + (int64_t)(b == 0 ? l2 * l2 : l2 * l2 + 2 * b - 1) * LD;
+      const double v = d[lay.rot_at(l2, 0, b, m)] * ((m + b) & 1 ? -1.0 : 1.0);
+      const double vr = cs[2 * b] * v, vi = sin_in * cs[2 * b + 1] * v;
+      const double* Ar = A + (int64_t)(b == 0 ? l2 * l2 : l2 * l2 + 2 * b - 1) * lda;
       double col = 0;
       for (int a = 0; a <= l; ++a) {
         const int ra = a == 0 ? l * l : l * l + 2 * a - 1;
         double re = Ar[ra] * vr, im = a ? Ar[ra + 1] * vr : 0.0;
         if (b) {
-          re += Ar[LD + ra] * vi;
-          im += a ? Ar[LD + ra + 1] * vi : 0.0;
+          re += Ar[lda + ra] * vi;
+          im += a ? Ar[lda + ra + 1] * vi : 0.0;
         }
-        col += d[lay.re_col(l, a) + m] * (cs[2 * a] * re + cs[2 * a + 1] * im);
+        col += d[lay.rot_at(l, 0, m, a)] * (cs[2 * a] * re + sin_out * cs[2 * a + 1] * im);
       }
       sum += col;
     }
-    // column l2 − m, row l − m of the block of order m
-    T[lay.offt[m] + (l2 - m) * rot_pad(p + 1 - m) + (l - m)] = m & 1 ? -sum : sum;
+    T[lay.trans_at(m, l - m, l2 - m)] = m & 1 ? -sum : sum;
   }
 }
 
@@ -98,142 +108,146 @@ __device__ __forceinline__ double flip(double x, int mask) {   // −x where mas
   return __hiloint2double(__double2hiint(x) ^ mask, __double2loint(x));
 }
 
-// y[i] += col[i]·x over a column of S coefficients on 16 bytes
-template <int S>
-__device__ __forceinline__ void axpy_column(double (&y)[S], const double* col, double x) {
-#pragma unroll
-  for (int i = 0; i < S; i += 2) {
-    const double2 b = *reinterpret_cast<const double2*>(col + i);
-    y[i] = fma(b.x, x, y[i]);
-    if (i + 1 < S) y[i + 1] = fma(b.y, x, y[i + 1]);
-  }
+// one FP64 tensor-core MMA, D(8×8) += A(8×4)·B(4×8): this lane holds A[g][t], B[t][g] and
+// D[g][2t], D[g][2t+1] (g = lane / 4, t = lane % 4)
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
 }
 
-// the rotation of degree L of this lane's C pairs, in place in their tile rows r (32·PT apart);
-// D: the degree's coefficients; cs: the pairs' (cos mφ, sin mφ), NC apart per order; BACK: the z
-// rotation after the product (to the offset's azimuth) instead of before it
-template <int L, int C, bool BACK>
-__device__ __forceinline__ void rotate_degree(double* r, int PT, const double* __restrict__ D,
-                                              const double2* __restrict__ cs, const int (&down)[C]) {
-  constexpr int NC = 32 * C, SR = rot_pad(L + 1), SI = rot_pad(L), K0 = L * L;
-  double yr[C][L + 1], yi[C][L > 0 ? L : 1];
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-#pragma unroll
-    for (int i = 0; i <= L; ++i) yr[c][i] = 0.0;
-#pragma unroll
-    for (int i = 0; i < L; ++i) yi[c][i] = 0.0;
-  }
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    double x = r[32 * c * PT + K0];
-    if (!BACK && (L & 1)) x = flip(x, down[c]);
-    axpy_column<L + 1>(yr[c], D, x);
-  }
-  if constexpr (L > 0) {
-    const double* col = D + SR;
-#pragma unroll 1
-    for (int k = 1; k <= L; ++k, col += SR + SI) {
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        double xr = r[32 * c * PT + K0 + 2 * k - 1], xi = r[32 * c * PT + K0 + 2 * k];
-        if (!BACK) {
-          double2 z = cs[k * NC + 32 * c];
-          if (L & 1) { z.x = flip(z.x, down[c]); z.y = flip(z.y, down[c]); }
-          const double t = z.x * xr - z.y * xi;
-          // the imaginary parts negated: Tᵐ acts on them with the opposite sign
-          xi = -(z.y * xr + z.x * xi);
-          xr = t;
-        }
-        axpy_column<L + 1>(yr[c], col, xr);
-        axpy_column<L>(yi[c], col + SR, xi);
-      }
-    }
-  }
-#pragma unroll
-  for (int c = 0; c < C; ++c) {
-    double* q = r + 32 * c * PT + K0;
-    const int dn = L & 1 ? down[c] : 0;
-    q[0] = BACK && (L & 1) ? flip(yr[c][0], dn) : yr[c][0];
-#pragma unroll
-    for (int j = 1; j <= L; ++j) {
-      double a = yr[c][j], b = yi[c][j - 1];
-      if (BACK) {
-        double2 z = cs[j * NC + 32 * c];
-        if (L & 1) { z.x = flip(z.x, dn); z.y = flip(z.y, dn); }
-        const double u = z.x * a - z.y * b, v = z.y * a + z.x * b;
-        a = j & 1 ? -u : u;                              // Σ
-        b = j & 1 ? -v : v;
-      }
-      q[2 * j - 1] = a;
-      q[2 * j] = b;
-    }
-  }
-}
-
-// the translation of order m over the S = p + 1 − m degrees m..p, in place; B the order's coefficients
-template <int S, int C>
-__device__ __forceinline__ void translate_order(double* r, int PT, int m, const double* __restrict__ B) {
-  constexpr int SP = rot_pad(S);
-  const int k0 = m * m + (m ? 2 * m - 1 : 0);            // degree l at l² + 2m − 1 (l² for m = 0)
-  double yr[C][S], yi[C][S];
-#pragma unroll
-  for (int c = 0; c < C; ++c)
-#pragma unroll
-    for (int i = 0; i < S; ++i) yr[c][i] = yi[c][i] = 0.0;
-  int k = k0, step = 2 * m + 1;
-  if (m == 0) {
-#pragma unroll 2
-    for (int i = 0; i < S; ++i, k += step, step += 2)
-#pragma unroll
-      for (int c = 0; c < C; ++c) axpy_column<S>(yr[c], B + i * SP, r[32 * c * PT + k]);
-  } else {
-#pragma unroll 1
-    for (int i = 0; i < S; ++i, k += step, step += 2)
-#pragma unroll
-      for (int c = 0; c < C; ++c) {
-        axpy_column<S>(yr[c], B + i * SP, r[32 * c * PT + k]);
-        axpy_column<S>(yi[c], B + i * SP, r[32 * c * PT + k + 1]);
-      }
-  }
-  k = k0;
-  step = 2 * m + 1;
-#pragma unroll
-  for (int i = 0; i < S; ++i) {
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      r[32 * c * PT + k] = yr[c][i];
-      if (m) r[32 * c * PT + k + 1] = yi[c][i];
-    }
-    k += step;
-    step += 2;
-  }
-}
-
-// the instance of a runtime degree or block size
-template <int L, int C, bool BACK>
-__device__ __forceinline__ void rotate_any(int l, double* r, int PT, const double* D, const double2* cs, const int (&down)[C]) {
-  if constexpr (L > 0) {
-    if (l < L) { rotate_any<L - 1, C, BACK>(l, r, PT, D, cs, down); return; }
-  }
-  rotate_degree<L, C, BACK>(r, PT, D, cs, down);
-}
-template <int S, int C>
-__device__ __forceinline__ void translate_any(int s, double* r, int PT, int m, const double* B) {
-  if constexpr (S > 1) {
-    if (s < S) { translate_any<S - 1, C>(s, r, PT, m, B); return; }
-  }
-  translate_order<S, C>(r, PT, m, B);
-}
-
-// an odd row length: the lanes' rows (columns of the tile) are free of bank conflicts
-__host__ __device__ constexpr int rot_row(int p) { return (p + 1) * (p + 1) | 1; }
+// The tile's row of one pair: degree l from base(l) on, the l + 1 real parts of m = 0..l, then the l
+// imaginary parts; base(l) ≡ l (mod 4) and a row is an odd multiple of 4 doubles, so that the 8 pairs ×
+// 4 orders (or 4 degrees of one order) a warp reads or writes at once lie in distinct banks
+__host__ __device__ constexpr int rot_base(int l) { return l * l + 2 * (l / 2); }
+__host__ __device__ constexpr int rot_row(int p) { return (rot_base(p + 1) + 3) / 4 * 4 | 4; }
+// the row of the pair's (cos mφ, sin mφ): zeros past m = p for the padded inputs
+__host__ __device__ constexpr int rot_cs(int p) { return (p + 4) / 8 * 8 + 5; }
 constexpr int rot_list(int nc) { return 4 * nc + 2; }   // source, offset (bit 31: it points down), target, runs; the last run's end, their count
 
-size_t rot_smem(const RotLayout& l, int C, int G) {
-  const int nc = 32 * C;
-  return sizeof(double) * ((size_t)l.nd + G * l.nt + (size_t)G * 2 * (l.p + 1) * nc + (size_t)G * nc * rot_row(l.p)) +
+size_t rot_smem(const RotLayout& l, int NG, int G) {
+  const int nc = 8 * NG;
+  return sizeof(double) * ((size_t)32 * (l.nd + G * l.nt) + (size_t)G * nc * (2 * rot_cs(l.p) + rot_row(l.p)) + 8) +
          sizeof(int) * (size_t)G * 2 * rot_list(nc);
+}
+
+// the rotation of degree l of NG groups of 8 pairs, in place: r, cs: this lane's pair of the first
+// group (pair g), PT and PM apart per pair; B: the degree's fragments at this lane; down: per group
+// the sign bit where the pair's offset points down; BACK: the z rotation after the product (to the
+// offset's azimuth) instead of before it. The imaginary parts of multipoles are negated on the way in
+// (not in ROT_L2L, whose inputs are locals) and on the way out where the output is one (ROT_M2M):
+// Tᵐ then acts on the real and the imaginary parts alike.
+template <int MODE, int RT, int NG, bool BACK>
+__device__ __forceinline__ void rotate_degree(int l, int t, double* r, int PT, const double2* cs, int PM,
+                                              const double* __restrict__ B, const int (&down)[NG]) {
+  double ar[NG][RT][2], ai[NG][RT][2];
+#pragma unroll
+  for (int q = 0; q < NG; ++q)
+#pragma unroll
+    for (int i = 0; i < RT; ++i) ar[q][i][0] = ar[q][i][1] = ai[q][i][0] = ai[q][i][1] = 0.0;
+  double* re = r + rot_base(l);
+  double* im = re + l;                                   // the imaginary part of m at im[m]
+  const int odd = l & 1;
+#pragma unroll 1
+  for (int k = t; k - t <= l; k += 4, B += 64 * RT) {
+    double br[RT], bi[RT];
+#pragma unroll
+    for (int i = 0; i < RT; ++i) { br[i] = B[64 * i]; bi[i] = B[64 * i + 32]; }
+#pragma unroll
+    for (int q = 0; q < NG; ++q) {
+      double xr = re[8 * q * PT + k], xi = im[8 * q * PT + k];
+      if (!BACK) {
+        double2 z = cs[8 * q * PM + k];
+        if (odd) { z.x = flip(z.x, down[q]); z.y = flip(z.y, down[q]); }
+        const double x = MODE == ROT_L2L ? -xi : xi, u = z.x * xr - z.y * x;
+        xi = -(z.y * xr + z.x * x);
+        xr = u;
+      }
+#pragma unroll
+      for (int i = 0; i < RT; ++i) {
+        dmma(ar[q][i], xr, br[i]);
+        dmma(ai[q][i], xi, bi[i]);
+      }
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int q = 0; q < NG; ++q)
+#pragma unroll
+    for (int i = 0; i < RT; ++i)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        const int m = 8 * i + t + 4 * e;
+        double a = ar[q][i][e], b = ai[q][i][e];
+        if (BACK && m <= l) {
+          double2 z = cs[8 * q * PM + m];
+          if (odd) { z.x = flip(z.x, down[q]); z.y = flip(z.y, down[q]); }
+          const int sg = (m & 1) << 31;                  // Σ
+          const double u = z.x * a - z.y * b, v = z.y * a + z.x * b;
+          a = flip(u, sg);
+          b = flip(MODE == ROT_M2M ? -v : v, sg);
+        }
+        if (m <= l) re[8 * q * PT + m] = a;
+        if (m <= l && m > 0) im[8 * q * PT + m] = b;
+      }
+}
+
+// the translation of order m over the degrees m..p, in place
+template <int RT, int NG>
+__device__ __forceinline__ void translate_order(int m, int p, int t, double* r, int PT, const double* __restrict__ B) {
+  double ar[NG][RT][2], ai[NG][RT][2];
+#pragma unroll
+  for (int q = 0; q < NG; ++q)
+#pragma unroll
+    for (int i = 0; i < RT; ++i) ar[q][i][0] = ar[q][i][1] = ai[q][i][0] = ai[q][i][1] = 0.0;
+#pragma unroll 1
+  for (int l0 = m; l0 <= p; l0 += 4, B += 32 * RT) {
+    const int l = min(l0 + t, p);                        // past p: zero coefficients
+    const double* x = r + rot_base(l) + m;
+    const int im = m ? l : 0;                            // m = 0 has no imaginary parts
+    double b[RT];
+#pragma unroll
+    for (int i = 0; i < RT; ++i) b[i] = B[32 * i];
+#pragma unroll
+    for (int q = 0; q < NG; ++q) {
+      const double xr = x[8 * q * PT], xi = x[8 * q * PT + im];
+#pragma unroll
+      for (int i = 0; i < RT; ++i) {
+        dmma(ar[q][i], xr, b[i]);
+        if (m) dmma(ai[q][i], xi, b[i]);
+      }
+    }
+  }
+  __syncwarp();
+#pragma unroll
+  for (int i = 0; i < RT; ++i)
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const int l = m + 8 * i + t + 4 * e;
+      if (l <= p) {
+        double* y = r + rot_base(l) + m;
+#pragma unroll
+        for (int q = 0; q < NG; ++q) {
+          y[8 * q * PT] = ar[q][i][e];
+          if (m) y[8 * q * PT + l] = ai[q][i][e];
+        }
+      }
+    }
+}
+
+template <int MODE, int TMAX, int NG, bool BACK>
+__device__ __forceinline__ void rotate_any(int l, int t, double* r, int PT, const double2* cs, int PM, const double* B,
+                                           const int (&down)[NG]) {
+  if (l < 8) rotate_degree<MODE, 1, NG, BACK>(l, t, r, PT, cs, PM, B, down);
+  else if (TMAX < 3 || l < 16) rotate_degree<MODE, 2, NG, BACK>(l, t, r, PT, cs, PM, B, down);
+  else rotate_degree<MODE, TMAX < 3 ? 2 : 3, NG, BACK>(l, t, r, PT, cs, PM, B, down);
+}
+template <int TMAX, int NG>
+__device__ __forceinline__ void translate_any(int m, int p, int t, double* r, int PT, const double* B) {
+  const int s = p + 1 - m;
+  if (s <= 8) translate_order<1, NG>(m, p, t, r, PT, B);
+  else if (TMAX < 3 || s <= 16) translate_order<2, NG>(m, p, t, r, PT, B);
+  else translate_order<TMAX < 3 ? 2 : 3, NG>(m, p, t, r, PT, B);
 }
 
 __device__ __forceinline__ void cpa16(void* dst, const void* src) {
@@ -245,37 +259,79 @@ __device__ __forceinline__ void cpa8(void* dst, const void* src) {
                : "memory");
 }
 
-// NW warps per group; LMAX ≥ p the largest degree
-template <int C, int G, int NW, int LMAX, int MINB>
-__global__ void __launch_bounds__(32 * NW * G, MINB)
-    k_m2l_rot(const __grid_constant__ RotSched sch, int nparts, int sub, int TB, const int4* __restrict__ blocks,
-              const int* __restrict__ cls_off, const int* __restrict__ rtab, const int2* __restrict__ pairs, const double* __restrict__ dtab,
-              const double2* __restrict__ csf, const uint64_t* __restrict__ lv_trans, const double* __restrict__ m2l_scale,
-              int LD, const double* __restrict__ M, double* __restrict__ Pl, int64_t pitch, int stokes) {
-  constexpr int NC = 32 * C, NT = 32 * NW, NL = rot_list(NC);
-  const int p = sch.lay.p, NP = (p + 1) * (p + 1), PT = rot_row(p), nd = sch.lay.nd, nt = sch.lay.nt;
+struct RotArgs {
+  RotSched sch;
+  const double* dtab;                   // the rotations' fragments by class
+  const double2* cst;                   // per far offset, or child slot, (cos mφ, sin mφ)
+  int LD, stokes;
+  int64_t pitch;
+  const double* in;                     // multipoles (the parents' locals for ROT_L2L)
+  double* out;                          // locals (the parents' multipoles for ROT_M2M)
+  // ROT_M2L: the blocks, `sub` parts of TB / sub targets each, and per level the translations
+  int nparts, sub, TB;
+  const int4* blocks;
+  const int *cls_off, *rtab;
+  const int2* pairs;
+  const uint64_t* lv_trans;
+  const double* m2l_scale;
+  // ROT_M2M, ROT_L2L: the level's sibling groups (children c0 .., eight each, of the parents gp), a
+  // multiple of eight children per CTA, the translation
+  int c0, nchild, per;
+  const int* gp;
+  const double* trans;
+};
+
+// NG groups of 8 pairs per chunk, G groups of NW warps; TMAX: 8-output tiles of the largest block;
+// NE: 32-entry pieces of an expansion
+template <int MODE, int NG, int G, int NW, int TMAX, int NE, int MINB>
+__global__ void __launch_bounds__(32 * NW * G, MINB) k_rot(const __grid_constant__ RotArgs A) {
+  static_assert(MODE == ROT_M2L || G == 1, "one group of warps per CTA in the sweeps");
+  const RotSched& sch = A.sch;
+  constexpr int NC = 8 * NG, NT = 32 * NW, NL = rot_list(NC);
+  const int p = sch.lay.p, NP = (p + 1) * (p + 1), PT = rot_row(p), PM = rot_cs(p), nd = 32 * sch.lay.nd, nt = 32 * sch.lay.nt;
   const int tid = threadIdx.x % NT, grp = threadIdx.x / NT, warp = tid >> 5, lane = tid & 31;
-  const int comp = blockIdx.y, psi = stokes && comp == 3;
+  const int comp = blockIdx.y, psi = A.stokes && comp == 3, LD = A.LD;
+  const int64_t pitch = A.pitch;
   extern __shared__ __align__(16) double sm[];
   double* D = sm;                                        // the class's rotation
   double* T = D + nd + grp * nt;                         // the group's translation
-  double2* cs = (double2*)(D + nd + G * nt) + (size_t)grp * (p + 1) * NC;   // [order][pair]
-  double* tile = (double*)((double2*)(D + nd + G * nt) + (size_t)G * (p + 1) * NC) + (size_t)grp * NC * PT;
-  int* list = (int*)((double*)((double2*)(D + nd + G * nt) + (size_t)G * (p + 1) * NC) + (size_t)G * NC * PT) + grp * 2 * NL;
+  double2* cs0 = (double2*)(D + nd + G * nt);
+  double2* cs = cs0 + (size_t)grp * NC * PM;             // [pair][order]
+  double* tile0 = (double*)(cs0 + (size_t)G * NC * PM);
+  double* tile = tile0 + (size_t)grp * NC * PT;          // [pair][entry], 8 doubles past the last row
+  int* list = (int*)(tile0 + (size_t)G * NC * PT + 8) + grp * 2 * NL;
+  // the padding stays zero: it meets zero coefficients
+  for (int i = threadIdx.x; i < G * NC * (2 * PM + PT) + 8; i += NT * G) ((double*)cs0)[i] = 0.0;
+  __syncthreads();
+  // where this lane's entries e = lane + 32k of an expansion lie in a row
+  int loc[NE];
+#pragma unroll
+  for (int k = 0; k < NE; ++k) {
+    int n, m, part;
+    coef_nmp(lane + 32 * k, n, m, part);
+    loc[k] = rot_base(n) + m + (part == 2 ? n : 0);
+  }
   auto gsync = [&] {
     if constexpr (G == 1) __syncthreads();
     else asm volatile("bar.sync %0, %1;" ::"r"(1 + grp), "n"(NT) : "memory");
   };
   // part q of block blk: its targets [t0, t1), whose pairs are consecutive in every class
-  const int part = blockIdx.x * G + grp, blk = part / sub, t0 = (part % sub) * (TB / sub), t1 = t0 + TB / sub;
-  const bool on = part < nparts;
-  const int4 b = on ? blocks[blk] : make_int4(0, 0, 0, 0);
-  const int level = b.x & 255;
-  const double alpha = on ? m2l_scale[level] : 0.0;
-  const int* co = cls_off + (int64_t)(on ? blk : 0) * (NCLASS + 1);
-  const double* lt = reinterpret_cast<const double*>(lv_trans[level]);
-  const double* Mc = M + (int64_t)comp * LD;
-  double* Pc = Pl + (int64_t)b.y * pitch + (int64_t)comp * LD;
+  const int part = blockIdx.x * G + grp;
+  const bool on = MODE != ROT_M2L || part < A.nparts;
+  int blk = 0, t0 = 0, t1 = 0;
+  int4 b = make_int4(0, 0, 0, 0);
+  double alpha = 1.0;
+  const double* lt = A.trans;
+  if constexpr (MODE == ROT_M2L) {
+    blk = part / A.sub;
+    t0 = part % A.sub * (A.TB / A.sub);
+    t1 = t0 + A.TB / A.sub;
+    if (on) b = A.blocks[blk];
+    alpha = on ? A.m2l_scale[b.x & 255] : 0.0;
+    lt = reinterpret_cast<const double*>(A.lv_trans[b.x & 255]);
+  }
+  const double* Mc = A.in + (int64_t)comp * LD;
+  double* Pc = A.out + (int64_t)b.y * pitch + (int64_t)comp * LD;
 
   // pair j of a list: its multipole into the tile's row j, its azimuth's table into the columns j
   auto gather = [&](const int* L, int j) {
@@ -283,46 +339,73 @@ __global__ void __launch_bounds__(32 * NW * G, MINB)
     const int f = L[NC + j] & 0xffff;
     const double* src = Mc + (int64_t)L[j] * pitch;
     if (psi) {
-      // the Stokes Ψ̂ block: its source is Ψ̂ + o·Φ of the source box, o the far offset
-      // (harmonics_stokes.jl: M2L Ψ̂_B = Ψ̂_A + o·Φ, linear in the source)
-      const double* phi = M + (int64_t)L[j] * pitch;
-      const double o0 = c_faroff[3 * f], o1 = c_faroff[3 * f + 1], o2 = c_faroff[3 * f + 2];
-      for (int e = lane; e < NP; e += 32)
-        row[e] = fma(o2, __ldg(phi + 2 * LD + e), fma(o1, __ldg(phi + LD + e), fma(o0, __ldg(phi + e), __ldg(src + e))));
+      // the Stokes Ψ̂ block takes Ψ̂ + o·Φ of a far box at offset o, ½Ψ̂ + δ̂·Φ of a child and
+      // 2Ψ̂ − 2δ̂·Φ of a parent, δ̂ the child's offset (harmonics_stokes.jl:77-129)
+      const double* phi = A.in + (int64_t)L[j] * pitch;
+      double o[3], c = MODE == ROT_M2M ? 0.5 : (MODE == ROT_L2L ? 2.0 : 1.0);
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        if (MODE == ROT_M2L) o[d] = c_faroff[3 * f + d];
+        else o[d] = (f >> d & 1 ? 0.25 : -0.25) * (MODE == ROT_L2L ? -2.0 : 1.0);
+      }
+#pragma unroll
+      for (int k = 0; k < NE; ++k) {
+        const int e = lane + 32 * k;
+        if (e < NP)
+          row[loc[k]] = fma(o[2], __ldg(phi + 2 * LD + e),
+                            fma(o[1], __ldg(phi + LD + e), fma(o[0], __ldg(phi + e), c * __ldg(src + e))));
+      }
     } else {
-      for (int e = lane; e < NP; e += 32) cpa8(row + e, src + e);
+#pragma unroll
+      for (int k = 0; k < NE; ++k)
+        if (lane + 32 * k < NP) cpa8(row + loc[k], src + lane + 32 * k);
     }
-    for (int m = lane; m <= p; m += 32) cpa16(cs + m * NC + j, csf + f * (p + 1) + m);
+    if (lane <= p) cpa16(cs + j * PM + lane, A.cst + f * (p + 1) + lane);
   };
   // the chunk's pairs read by the group's first warp, then into the list with the runs of one target
   // (the pairs of a class are grouped by target)
-  auto fetch = [&](int q0, int nc, int2 (&pr)[C]) {
-#pragma unroll
-    for (int c = 0; c < C; ++c) pr[c] = 32 * c + lane < nc ? pairs[b.w + q0 + 32 * c + lane] : make_int2(0, -1);
-  };
-  auto commit = [&](int* L, int nc, const int2 (&pr)[C]) {
-    int base = 0, last = -1;
-#pragma unroll
-    for (int c = 0; c < C; ++c) {
-      const int j = 32 * c + lane, tg = pr[c].y < 0 ? -1 : pr[c].y & 0xff;
-      int prev = __shfl_up_sync(0xffffffffu, tg, 1);
-      if (lane == 0) prev = last;
-      last = __shfl_sync(0xffffffffu, tg, 31);
-      const bool start = j < nc && tg != prev;
-      const unsigned bal = __ballot_sync(0xffffffffu, start);
-      L[j] = pr[c].x;
-      const int f = pr[c].y < 0 ? 0 : pr[c].y >> 8;
-      L[NC + j] = f | (c_faroff[3 * f + 2] < 0) << 31;
-      L[2 * NC + j] = tg;
-      if (start) L[3 * NC + base + __popc(bal & ((1u << lane) - 1u))] = j;
-      base += __popc(bal);
+  auto fetch = [&](int q0, int nc) {                     // source, offset or child slot, target (−1: none)
+    if (lane >= nc) return make_int3(0, 0, -1);
+    const int q = q0 + lane;
+    if constexpr (MODE == ROT_M2L) {
+      const int2 pr = A.pairs[b.w + q];
+      return make_int3(pr.x, pr.y >> 8, pr.y & 0xff);
+    } else {
+      const int c = A.c0 + q, pa = A.gp[q >> 3];
+      return MODE == ROT_M2M ? make_int3(c, q & 7, pa) : make_int3(pa, q & 7, c);
     }
-    if (lane == 0) { L[3 * NC + base] = nc; L[4 * NC + 1] = base; }
   };
+  auto commit = [&](int* L, int nc, int3 pr) {
+    const int prev = __shfl_up_sync(0xffffffffu, pr.z, 1);
+    const bool start = lane < nc && (lane == 0 || pr.z != prev);
+    const unsigned bal = __ballot_sync(0xffffffffu, start);
+    if (lane < NC) {
+      const bool down = MODE == ROT_M2L ? c_faroff[3 * pr.y + 2] < 0 : !(pr.y >> 2);
+      L[lane] = pr.x;
+      L[NC + lane] = pr.y | (int)down << 31;
+      L[2 * NC + lane] = pr.z;
+    }
+    if (start) L[3 * NC + __popc(bal & ((1u << lane) - 1u))] = lane;
+    if (lane == 0) { L[3 * NC + __popc(bal)] = nc; L[4 * NC + 1] = __popc(bal); }
+  };
+  static_assert(NC <= 32, "a lane per pair of a chunk");
+  const int g = lane >> 2, t = lane & 3;
+  double* row0 = tile + g * PT;                          // this lane's pair of the first 8
+  const double2* cs_g = cs + g * PM;
 
-  for (int c = 0; c < NCLASS; ++c) {
-    const int* rt = rtab + ((int64_t)blk * NCLASS + c) * TB;
-    const int a0 = on ? co[c] + (t0 ? rt[t0] & 0xffff : 0) : 0, a1 = on ? (t1 < TB ? co[c] + (rt[t1] & 0xffff) : co[c + 1]) : 0;
+  for (int c = 0; c < (MODE == ROT_M2L ? NCLASS : 1); ++c) {
+    int a0 = 0, a1 = 0;
+    if constexpr (MODE == ROT_M2L) {
+      const int* co = A.cls_off + (int64_t)(on ? blk : 0) * (NCLASS + 1);
+      const int* rt = A.rtab + ((int64_t)blk * NCLASS + c) * A.TB;
+      if (on) {
+        a0 = co[c] + (t0 ? rt[t0] & 0xffff : 0);
+        a1 = t1 < A.TB ? co[c] + (rt[t1] & 0xffff) : co[c + 1];
+      }
+    } else {
+      a0 = part * A.per;
+      a1 = min(A.nchild, a0 + A.per);
+    }
     if constexpr (G == 1) {
       if (a0 == a1) continue;
     } else {
@@ -330,16 +413,14 @@ __global__ void __launch_bounds__(32 * NW * G, MINB)
     }
     // the class's tables, the first chunk's list and multipoles
     {
-      const double* src = dtab + (int64_t)c * nd;
+      const double* src = A.dtab + (int64_t)(MODE == ROT_M2L ? c : NCLASS) * nd;
       for (int i = 2 * threadIdx.x; i < nd; i += 2 * NT * G) cpa16(D + i, src + i);
       const double* ts = lt + (int64_t)c * nt;
       if (a0 < a1)                                       // an idle group has no level
         for (int i = 2 * tid; i < nt; i += 2 * NT) cpa16(T + i, ts + i);
     }
     if (warp == 0 && a0 < a1) {
-      int2 pr[C];
-      fetch(a0, min(NC, a1 - a0), pr);
-      commit(list, min(NC, a1 - a0), pr);
+      commit(list, min(NC, a1 - a0), fetch(a0, min(NC, a1 - a0)));
     }
     gsync();
     for (int j = warp; j < min(NC, a1 - a0); j += NW) gather(list, j);
@@ -350,28 +431,28 @@ __global__ void __launch_bounds__(32 * NW * G, MINB)
       const int* L = list + cur * NL;
       int* Ln = list + (cur ^ 1) * NL;
       const int nn = min(NC, a1 - q0 - NC);              // the next chunk's pairs (≤ 0: none in this class)
-      int2 pr[C];
-      if (warp == 0 && nn > 0) fetch(q0 + NC, nn, pr);
-      int down[C];
+      int3 pr;
+      if (warp == 0 && nn > 0) pr = fetch(q0 + NC, nn);
+      int down[NG];
 #pragma unroll
-      for (int k = 0; k < C; ++k) down[k] = L[NC + 32 * k + lane] & (int)0x80000000;
+      for (int k = 0; k < NG; ++k) down[k] = L[NC + 8 * k + g] & (int)0x80000000;
 #pragma unroll 1
       for (int i = sch.first[0][warp]; i < sch.first[0][warp + 1]; ++i) {
         const int l = sch.order[0][i];
-        rotate_any<LMAX, C, false>(l, tile + lane * PT, PT, D + sch.lay.offd[l], cs + lane, down);
+        rotate_any<MODE, TMAX, NG, false>(l, t, row0, PT, cs_g, PM, D + 32 * sch.lay.offd[l] + lane, down);
       }
       if (warp == 0 && nn > 0) commit(Ln, nn, pr);
       gsync();
 #pragma unroll 1
       for (int i = sch.first[1][warp]; i < sch.first[1][warp + 1]; ++i) {
         const int m = sch.order[1][i];
-        translate_any<LMAX + 1, C>(p + 1 - m, tile + lane * PT, PT, m, T + sch.lay.offt[m]);
+        translate_any<TMAX, NG>(m, p, t, row0, PT, T + 32 * sch.lay.offt[m] + lane);
       }
       gsync();
 #pragma unroll 1
       for (int i = sch.first[0][warp]; i < sch.first[0][warp + 1]; ++i) {
         const int l = sch.order[0][i];
-        rotate_any<LMAX, C, true>(l, tile + lane * PT, PT, D + sch.lay.offd[l], cs + lane, down);
+        rotate_any<MODE, TMAX, NG, true>(l, t, row0, PT, cs_g, PM, D + 32 * sch.lay.offd[l] + lane, down);
       }
       gsync();
       // scatter: a warp the runs w, w + NW, ..., the entries across the lanes; then the next chunk's
@@ -380,18 +461,17 @@ __global__ void __launch_bounds__(32 * NW * G, MINB)
       for (int r = warp; r < nrun; r += NW) {
         const int j0 = L[3 * NC + r], j1 = L[3 * NC + r + 1];
         double* dst = Pc + (int64_t)L[2 * NC + j0] * pitch;
-        for (int e0 = lane; e0 < NP; e0 += 128) {
-          double v[4];
+        // a parent's multipole starts from zero: its eight children are one run
+        double v[NE];
 #pragma unroll
-          for (int k = 0; k < 4; ++k) v[k] = e0 + 32 * k < NP ? dst[e0 + 32 * k] : 0.0;
-          for (int j = j0; j < j1; ++j)
+        for (int k = 0; k < NE; ++k) v[k] = MODE != ROT_M2M && lane + 32 * k < NP ? dst[lane + 32 * k] : 0.0;
+        for (int j = j0; j < j1; ++j)
 #pragma unroll
-            for (int k = 0; k < 4; ++k)
-              if (e0 + 32 * k < NP) v[k] = fma(alpha, tile[j * PT + e0 + 32 * k], v[k]);
+          for (int k = 0; k < NE; ++k)
+            if (lane + 32 * k < NP) v[k] = fma(alpha, tile[j * PT + loc[k]], v[k]);
 #pragma unroll
-          for (int k = 0; k < 4; ++k)
-            if (e0 + 32 * k < NP) dst[e0 + 32 * k] = v[k];
-        }
+        for (int k = 0; k < NE; ++k)
+          if (lane + 32 * k < NP) dst[lane + 32 * k] = v[k];
         if (nn > 0) {
           __syncwarp();
           for (int j = j0; j < min(j1, nn); ++j) gather(Ln, j);
@@ -408,12 +488,11 @@ RotSched schedule(const RotLayout& lay, int nw) {
   RotSched s{};
   s.lay = lay;
   for (int kind = 0; kind < 2; ++kind) {
-    // the work of degree l: (l + 1)² + l² products; of order m over q = p + 1 − m degrees: 2q² (q² for
-    // m = 0); and the rows read and written
+    // the MMAs of degree l, of order m (half of them for m = 0), and a task's fixed part
     std::vector<int> cost(lay.p + 1), id(lay.p + 1);
     for (int i = 0; i <= lay.p; ++i) {
-      const int q = lay.p + 1 - i;
-      cost[i] = kind == 0 ? (i + 1) * (i + 1) + i * i + 12 * i + 20 : (i ? 2 : 1) * q * (q + 6) + 20;
+      const int q = kind == 0 ? i + 1 : lay.p + 1 - i;
+      cost[i] = (kind == 1 && i == 0 ? 1 : 2) * RotLayout::ksteps(q) * RotLayout::tiles(q) + 2;
       id[i] = i;
     }
     std::stable_sort(id.begin(), id.end(), [&](int a, int b) { return cost[a] > cost[b]; });
@@ -436,49 +515,108 @@ RotSched schedule(const RotLayout& lay, int nw) {
 
 // The parts a block is cut into: more of them fill the device (`slots` groups run at once), fewer
 // of them fill the chunks (a class's last chunk of a part is half empty on average, and one with
-// few pairs costs a whole one): the power of two with the least waves × chunks per part. Measured
-// at 6.04M far pairs of 293 blocks, p = 10 (1, 2, 4, 8 parts): 7.9, 6.0, 6.0, 6.3 ms; at 207,331
-// pairs of a sphere: 0.77, 0.59, 0.72, 0.95 ms.
-int parts_per_block(const Plan& P, int nexp, int slots) {
+// few pairs costs a whole one): the power of two with the least waves × chunks per part. Measured with
+// the products on the FMA units at 6.04M far pairs of 293 blocks, p = 10 (1, 2, 4, 8 parts): 7.9, 6.0,
+// 6.0, 6.3 ms; at 207,331 pairs of a sphere: 0.77, 0.59, 0.72, 0.95 ms.
+int parts_per_block(const Plan& P, int nexp, int slots, int nc) {
   const double nb = (double)P.h_blocks.size();
   int best = 1;
   double least = 1e300;
   for (int sub = 1; sub <= P.TB / 4; sub *= 2) {
     const double pairs = (double)P.npairs / (nb * sub * NCLASS);
-    const double t = std::max(1.0, nb * sub * nexp / slots) * std::max(1.0, pairs / 32 + 0.5);
+    const double t = std::max(1.0, nb * sub * nexp / slots) * std::max(1.0, pairs / nc + 0.5);
     if (t < 0.97 * least) { least = t; best = sub; }
   }
   return best;
 }
 
-template <int C, int G, int NW, int LMAX, int MINB>
+template <int MODE, int NG, int G, int NW, int TMAX, int NE, int MINB>
+void start(RotArgs& A, const RotHost& R, int ctas, int nexp, cudaStream_t s) {
+  A.sch = schedule(R.layout, NW);
+  const size_t smem = rot_smem(R.layout, NG, G);
+  auto kern = k_rot<MODE, NG, G, NW, TMAX, NE, MINB>;
+  FMMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  kern<<<dim3(ctas, nexp), 32 * NW * G, smem, s>>>(A);
+  FMMB_LAUNCH_CHECK();
+}
+
+RotArgs common_args(State& S, const double* cst, const double* in, double* out) {
+  Cache& K = *S.plan->cache;
+  RotArgs A{};
+  A.dtab = K.rot_d.p;
+  A.cst = (const double2*)cst;
+  A.LD = K.ld;
+  A.stokes = K.nexp == 4;
+  A.pitch = (int64_t)K.nexp * K.ld;
+  A.in = in;
+  A.out = out;
+  return A;
+}
+
+template <int NG, int G, int NW, int TMAX, int NE, int MINB>
 void launch(State& S) {
   Plan& P = *S.plan;
   Cache& K = *P.cache;
   const int nb = (int)P.h_blocks.size();
   if (nb == 0) return;
-  const RotSched sch = schedule(K.rot->layout, NW);
-  const size_t smem = rot_smem(K.rot->layout, C, G);
-  auto kern = k_m2l_rot<C, G, NW, LMAX, MINB>;
-  FMMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  const int sub = parts_per_block(P, K.nexp, P.ctx->num_sms * MINB * G);
-  kern<<<dim3((nb * sub + G - 1) / G, K.nexp), 32 * NW * G, smem, P.ctx->stream>>>(
-      sch, nb * sub, sub, P.TB, P.blocks.p, P.cls_off.p, P.rtab.p, P.pairs.p, K.rot_d.p, (const double2*)K.rot_csf.p, P.d_lv_rot.p, P.d_m2l_scale.p,
-      K.ld, S.M.p, S.Pl.p, (int64_t)K.nexp * K.ld, K.nexp == 4);
-  FMMB_LAUNCH_CHECK();
+  RotArgs A = common_args(S, K.rot_csf.p, S.M.p, S.Pl.p);
+  A.sub = parts_per_block(P, K.nexp, P.ctx->num_sms * MINB * G, 8 * NG);
+  A.nparts = nb * A.sub;
+  A.TB = P.TB;
+  A.blocks = P.blocks.p;
+  A.cls_off = P.cls_off.p;
+  A.rtab = P.rtab.p;
+  A.pairs = P.pairs.p;
+  A.lv_trans = P.d_lv_rot.p;
+  A.m2l_scale = P.d_m2l_scale.p;
+  start<ROT_M2L, NG, G, NW, TMAX, NE, MINB>(A, *K.rot, (A.nparts + G - 1) / G, K.nexp, P.ctx->stream);
 }
 
-void translations(Cache& C, const RotLayout& lay, const double* reps, DBuf<double>& out, cudaStream_t s) {
-  out.alloc((size_t)NCLASS * lay.nt);
-  k_rot_translations<<<NCLASS, 256, 0, s>>>(reps, C.rot_d.p, C.rot_cs.p, lay, C.ld, out.p);
+// the children of level l (into their parents, or from them): chunks spread over the CTAs that run at once
+template <int MODE, int NG, int NW, int TMAX, int NE, int MINB>
+void launch_sweep(State& S, int l, const double* trans) {
+  Plan& P = *S.plan;
+  Cache& K = *P.cache;
+  RotArgs A = MODE == ROT_M2M ? common_args(S, K.rot_csk.p, S.M.p, S.M.p) : common_args(S, K.rot_csk.p, S.Pl.p, S.Pl.p);
+  A.c0 = P.level_start[l];
+  A.nchild = NCH * P.level_groups[l];
+  A.gp = P.group_parent[l].p;
+  A.trans = trans;
+  const int slots = std::max(1, P.ctx->num_sms * MINB / K.nexp), chunks = (A.nchild + 8 * NG - 1) / (8 * NG);
+  A.per = 8 * NG * ((chunks + slots - 1) / slots);
+  start<MODE, NG, 1, NW, TMAX, NE, MINB>(A, *K.rot, (A.nchild + A.per - 1) / A.per, K.nexp, P.ctx->stream);
+}
+
+template <int MODE>
+void sweep(State& S, int l, const double* trans) {
+  const int p = S.plan->cache->p;
+  if (p <= 11) launch_sweep<MODE, 3, 4, 2, 5, 4>(S, l, trans);
+  else if (p <= 15) launch_sweep<MODE, 3, 6, 2, 8, 2>(S, l, trans);
+  else if (p == 16) launch_sweep<MODE, 2, 8, 3, 10, 1>(S, l, trans);
+  else launch_sweep<MODE, 2, 8, 3, 14, 1>(S, l, trans);
+}
+
+// the translations along z of n classes (c0 ..) from their dense operators
+void translations(Cache& C, const RotLayout& lay, int mode, int c0, int n, const double* dense, int lda, int64_t stride,
+                  DBuf<double>& out, cudaStream_t s) {
+  out.alloc((size_t)n * 32 * lay.nt);
+  k_rot_translations<<<n, 256, 0, s>>>(dense, lda, stride, mode, c0, C.rot_d.p, C.rot_cs.p, lay, out.p);
   FMMB_LAUNCH_CHECK();
+}
+void all_translations(Cache& C, const RotLayout& lay, const double* reps, const double* m2m, const double* l2l,
+                      RotTrans& t, cudaStream_t s) {
+  const int LD = C.ld;
+  translations(C, lay, ROT_M2L, 0, NCLASS, reps, LD, (int64_t)LD * LD, t.m2l, s);
+  // of the child slot (1, 1, 1), the last: the direction the rotation is built for
+  translations(C, lay, ROT_M2M, NCLASS, 1, m2m + (int64_t)7 * LD * LD, LD, 0, t.m2m, s);
+  translations(C, lay, ROT_L2L, NCLASS, 1, l2l + (int64_t)7 * LD, NCH * LD, 0, t.l2l, s);
 }
 
 }  // namespace
 
-// the tables of the FP64 M2L: the cache's rotations (uploaded with its first FP64 state) and per
-// level the translations along z (the cache's for the homogeneous kernels, the level width's own
-// for Yukawa3D). The cache is locked by the caller.
+// the tables of the FP64 translations: the cache's rotations (uploaded with its first state) and per
+// level the translations along z (the cache's for the homogeneous kernels, the level width's own for
+// Yukawa3D). The cache is locked by the caller.
 void prepare_rotations(Plan& P) {
   Cache& C = *P.cache;
   cudaStream_t s = P.ctx->stream;
@@ -488,47 +626,62 @@ void prepare_rotations(Plan& P) {
     to_device(C.rot_d, h->d, s);
     to_device(C.rot_cs, h->cs, s);
     to_device(C.rot_csf, h->csf, s);
-    if (C.kernel != FMMB_KERNEL_YUKAWA3D) translations(C, h->layout, C.reps.p, C.rot_t, s);
+    to_device(C.rot_csk, h->csk, s);
+    if (C.kernel != FMMB_KERNEL_YUKAWA3D) all_translations(C, h->layout, C.reps.p, C.m2m.p, C.l2l.p, C.rot_t, s);
     C.rot = h;
   }
   std::vector<uint64_t> t(P.L, 0);
+  P.lv_rot_m2m.assign(P.L, nullptr);
+  P.lv_rot_l2l.assign(P.L, nullptr);
   for (int l = 0; l < P.L; ++l) {
+    const RotTrans* r = nullptr;
     if (C.kernel != FMMB_KERNEL_YUKAWA3D) {
-      t[l] = (uint64_t)(uintptr_t)C.rot_t.p;
+      r = &C.rot_t;
     } else if (l >= 2 && l < (int)P.lv_yukawa.size() && P.lv_yukawa[l]) {
       YukawaLevel& Y = *P.lv_yukawa[l];
       std::lock_guard<std::mutex> lk(Y.mu);
-      if (!Y.rot_t.n) {
+      if (!Y.rot_t.l2l.n) {
         // shared by caches on other streams: outside the stream-ordered pool, complete before use
         const cudaStream_t keep = g_alloc_stream;
         g_alloc_stream = nullptr;
         try {
-          translations(C, C.rot->layout, Y.reps.p, Y.rot_t, s);
+          all_translations(C, C.rot->layout, Y.reps.p, Y.m2m.p, Y.l2l.p, Y.rot_t, s);
           FMMB_CUDA(cudaStreamSynchronize(s));
         } catch (...) {
-          Y.rot_t.release();
+          Y.rot_t = RotTrans();
           g_alloc_stream = keep;
           throw;
         }
         g_alloc_stream = keep;
       }
-      t[l] = (uint64_t)(uintptr_t)Y.rot_t.p;
+      r = &Y.rot_t;
     }
+    if (!r) continue;                                    // no translations touch the level
+    t[l] = (uint64_t)(uintptr_t)r->m2l.p;
+    P.lv_rot_m2m[l] = r->m2m.p;
+    P.lv_rot_l2l[l] = r->l2l.p;
   }
   to_device(P.d_lv_rot, t, s);
 }
 
+// the children of level l + 1 into the parents of level l; the parents' locals of level l − 1 into the
+// children of level l
+void m2m_rot(State& S, int l) { sweep<ROT_M2M>(S, l + 1, S.plan->lv_rot_m2m[l]); }
+void l2l_rot(State& S, int l) { sweep<ROT_L2L>(S, l, S.plan->lv_rot_l2l[l - 1]); }
+
+// Chunks of 24 pairs and two to four CTAs per SM while the tiles and tables fit (400,000 points p = 10:
+// 5.42 ms, sphere of 30,000 0.49; chunks of 16 6.42 and 0.50; two groups with chunks of 32 5.50 and 0.65.
+// p = 14: 11.6; chunks of 16 14.4; four warps instead of six 13.8). At p = 16 one CTA fits: two groups of
+// warps share the rotations, one computing while the other scatters, as long as there are pairs enough
+// for that many chunks (6.04M pairs: 16.5 ms against 23.8 for one group; 1.05M: 3.83 against 4.31), one
+// group where there are not (71,365: 0.61 against 0.64; 56,448: 0.46 against 0.64).
 void m2l_rot(State& S) {
   const int p = S.plan->cache->p;
-  // four warps share a tile up to p = 13; above, the largest degree is a smaller share of the work and
-  // more warps even out. At p = 16 one tile and the class's tables take 122 KB: two groups share the
-  // tables (6.04M pairs: 15.0 ms, 20.0 ms with one), where there are enough blocks for both.
-  if (p <= 11) launch<1, 1, 4, 11, 4>(S);
-  else if (p <= 13) launch<1, 1, 4, 13, 3>(S);
-  else if (p <= 15) launch<1, 1, 6, 15, 2>(S);
-  else if (p == 16 && (int64_t)S.plan->h_blocks.size() * S.plan->cache->nexp >= 2 * S.plan->ctx->num_sms) launch<1, 2, 6, 16, 1>(S);
-  else if (p == 16) launch<1, 1, 8, 16, 1>(S);
-  else launch<1, 1, 8, 20, 1>(S);
+  if (p <= 11) launch<3, 1, 4, 2, 5, 4>(S);
+  else if (p <= 15) launch<3, 1, 6, 2, 8, 2>(S);
+  else if (p == 16 && (int64_t)S.plan->npairs * S.plan->cache->nexp >= 1000000) launch<3, 2, 6, 3, 10, 1>(S);
+  else if (p == 16) launch<2, 1, 8, 3, 10, 1>(S);
+  else launch<2, 1, 8, 3, 14, 1>(S);
 }
 
 }  // namespace fmmb

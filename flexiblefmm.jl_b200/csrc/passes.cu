@@ -409,11 +409,6 @@ void gemm_columns(int M, int K, const double* A, ColMap bm, ColMap cm, int ncols
   gemm_cols(M, K, A, bm, cm, ncols, LD, NP, accumulate, num_sms, s);
 }
 
-void gemm_expansions(int M, int K, const double* A, ColMap bm, ColMap cm, int ncols, int LD, int NP, int accumulate,
-                     int num_sms, cudaStream_t s) {
-  gemm_cols(M, K, A, bm, cm, ncols, LD, NP, accumulate, num_sms, s, LD, NP);
-}
-
 int p2m(State& S) {
   if (S.plan->cache->method == FMMB_METHOD_CUBE_KI) return ki_p2m(S);
   if (S.plan->cache->method == FMMB_METHOD_KI_CIRCLE) return kic_p2m(S);
@@ -430,9 +425,13 @@ int m2m_sweep(State& S) {
   for (int l = P.L - 2; l >= 2; --l) {
     int c0 = P.level_start[l + 1], ng = P.level_groups[l + 1];
     if (ng == 0) continue;
+    ++launches;
+    if (C.method == FMMB_METHOD_SPHERICAL_HARMONICS) {
+      m2m_rot(S, l);
+      continue;
+    }
     ColMap bm{S.M.p, nullptr, c0, NCH}, cm{S.M.p, P.group_parent[l + 1].p, 0, 0};
     gemm_cols(C.ld, NCH * C.ld, P.lv_m2m[l], bm, cm, ng, C.ld, C.np, 0, P.ctx->num_sms, s, C.ld, C.np);
-    ++launches;
   }
   return launches;
 }
@@ -466,12 +465,21 @@ int l2l_sweep(State& S) {
   Cache& C = *P.cache;
   cudaStream_t s = P.ctx->stream;
   int launches = 0;
+  // by rotations, or below order 8 (one expansion a node) as dense products, whose fewer steps then count
+  // for more than their multiplications (rotations against dense, 400,000 uniform points: p = 4 0.050
+  // against 0.042 ms, p = 7 0.058 against 0.050, p = 10 0.083 against 0.103; M2M is faster by rotations at
+  // every order: p = 2 0.040 against 0.044, p = 7 0.048 against 0.069)
+  const bool by_rotations = C.method == FMMB_METHOD_SPHERICAL_HARMONICS && (C.nexp == 4 || C.p >= 8);
   for (int l = 3; l < P.L; ++l) {
     int c0 = P.level_start[l], ng = P.level_groups[l];
     if (ng == 0) continue;
+    ++launches;
+    if (by_rotations) {
+      l2l_rot(S, l);
+      continue;
+    }
     ColMap bm{S.Pl.p, P.group_parent[l].p, 0, 0}, cm{S.Pl.p, nullptr, c0, NCH};
     gemm_cols(NCH * C.ld, C.ld, P.lv_l2l[l - 1], bm, cm, ng, C.ld, C.np, 1, P.ctx->num_sms, s, C.ld, C.np);
-    ++launches;
   }
   // the kernel-independent method: the leaves' local densities from their check potentials
   if (C.method == FMMB_METHOD_CUBE_KI) launches += ki_leaf_locals(S);

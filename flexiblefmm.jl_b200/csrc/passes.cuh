@@ -1,4 +1,4 @@
-// Declarations shared by the pass kernels (passes.cu, m2l_f64.cu, m2l_tc.cu, eval.cu).
+// Declarations shared by the pass kernels (passes.cu, p2m.cu, m2l_rot.cu, m2l_tc.cu, eval.cu).
 #pragma once
 #include "plan.cuh"
 
@@ -209,15 +209,13 @@ struct ColMap {
 // C(:, g) (=|+=) A · B(:, g) on the FP64 tensor cores; rows r with r mod LD ≥ NP written as 0
 void gemm_columns(int M, int K, const double* A, ColMap bm, ColMap cm, int ncols, int LD, int NP, int accumulate,
                   int num_sms, cudaStream_t s);
-// the same over expansions (K in blocks of LD whose entries k mod LD ≥ NP are zero columns of A:
-// M2M and L2L), without multiplying that padding
-void gemm_expansions(int M, int K, const double* A, ColMap bm, ColMap cm, int ncols, int LD, int NP, int accumulate,
-                     int num_sms, cudaStream_t s);
 // P2M of the childless sourced nodes (p2m.cu): nsets charge sets (tree order) and, all or none, dipoles
 // (3 × N planar) into the blocks at M[a], pitch doubles per node; returns the launches
 int p2m_blocks(State& S, int nsets, const double* const* q, const double* const* d3, double* const* M, int64_t pitch);
 
 void m2l_rot(State& S);
+void m2m_rot(State& S, int l);     // the children of level l + 1 into level l
+void l2l_rot(State& S, int l);     // level l − 1 into its children
 void prepare_rotations(Plan& P);   // the cache locked by the caller
 int p2m(State& S);          // the stages of the passes; each returns its kernel launches
 int m2m_sweep(State& S);

@@ -17,6 +17,9 @@ struct Ctx {
   int num_sms = 148;
 };
 
+// The translations along z of the FP64 M2L (34 classes), M2M and L2L (m2l_rot.cu)
+struct RotTrans { DBuf<double> m2l, m2m, l2l; };
+
 // The Yukawa operators of one box width (src/operators/harmonics_yukawa.jl:164-207): the 34
 // class representatives with c_K / w folded in, M2M (children of width w/2 into the parent) and
 // L2L (the parent into its children), in the Laplace layouts.
@@ -27,8 +30,8 @@ struct YukawaLevel {
   std::mutex mu;
   DBuf<uint16_t> reps16;
   DBuf<float> row_scale;
-  // the FP64 M2L's translations along z of this width (built when an FP64 state first needs them)
-  DBuf<double> rot_t;
+  // the FP64 translations along z of this width (built when a state first needs them)
+  RotTrans rot_t;
 };
 
 // OperatorCache (src/operators/cache.jl:5-83): the base width, the host operators at the base
@@ -53,10 +56,11 @@ struct Cache {
   DBuf<float> row_scale;
   DBuf<uint32_t> perm16;
   bool split_ready = false;
-  // the FP64 M2L (m2l_rot.cu): per class the rotation of its representative offset to the z axis
-  // and the translation along z (Yukawa3D: the level widths')
+  // the FP64 translations (m2l_rot.cu): per class the rotation of its representative offset to the z
+  // axis, and the translations along z (Yukawa3D: the level widths')
   std::shared_ptr<const RotHost> rot;
-  DBuf<double> rot_d, rot_cs, rot_csf, rot_t;
+  DBuf<double> rot_d, rot_cs, rot_csf, rot_csk;
+  RotTrans rot_t;
   // Yukawa3D: κ, the operators per width (keyed by the exponent e of w = ldexp(W0, e); built on
   // first use and shared by every cache of the same device, order, κ and width), and the sphere
   // quadrature of the projections
@@ -134,7 +138,10 @@ struct Plan {
   std::vector<const double*> lv_reps, lv_m2m, lv_l2l;
   DBuf<uint64_t> d_lv_reps;
   DBuf<double> d_kh2;
-  DBuf<uint64_t> d_lv_rot;                // the FP64 path: per level the translations along z of the classes
+  // per level the translations along z: of the classes (a table on the device), into the level's
+  // nodes from their children, out of the level's nodes into theirs
+  DBuf<uint64_t> d_lv_rot;
+  std::vector<const double*> lv_rot_m2m, lv_rot_l2l;
   // the mixed path: per level the split class operators and their inverse row scales (the cache's
   // for the homogeneous kernels, the level width's own for Yukawa3D), built with the first mixed
   // state; the Yukawa levels they come from stay held by the plan

@@ -49,18 +49,14 @@ void harmonics_at(ld x, ld y, ld z, int p, std::vector<ld>& vr, std::vector<ld>&
 RotLayout make_layout(int p) {
   RotLayout R;
   R.p = p;
-  int o = 0;
   for (int l = 0; l <= p; ++l) {
-    R.offd[l] = (uint16_t)o;
-    o += (l + 1) * rot_pad(l + 1) + l * rot_pad(l);
+    R.offd[l] = (uint16_t)R.nd;
+    R.nd += 2 * RotLayout::ksteps(l + 1) * RotLayout::tiles(l + 1);
   }
-  R.nd = o;
-  o = 0;
   for (int m = 0; m <= p; ++m) {
-    R.offt[m] = (uint16_t)o;
-    o += (p + 1 - m) * rot_pad(p + 1 - m);
+    R.offt[m] = (uint16_t)R.nt;
+    R.nt += RotLayout::ksteps(p + 1 - m) * RotLayout::tiles(p + 1 - m);
   }
-  R.nt = o;
   return R;
 }
 
@@ -98,7 +94,9 @@ void legendre_rule(int n, std::vector<T>& t, std::vector<T>& w, T pi, T eps) {
 }
 
 std::shared_ptr<const RotHost> build(int p, const HostOperators& op) {
-  const std::vector<int>& reps_off = op.reps_off;
+  // the classes of the far offsets, then the direction of the child slots
+  std::vector<int> reps_off = op.reps_off;
+  reps_off.insert(reps_off.end(), {1, 1, 1});
   auto H = std::make_shared<RotHost>();
   H->layout = make_layout(p);
   const RotLayout& R = H->layout;
@@ -124,7 +122,7 @@ std::shared_ptr<const RotHost> build(int p, const HostOperators& op) {
         }
     }
   const int ncls = (int)reps_off.size() / 3;
-  H->d.assign((size_t)ncls * R.nd, 0.0);
+  H->d.assign((size_t)ncls * 32 * R.nd, 0.0);
   H->cs.assign((size_t)ncls * 2 * (p + 1), 0.0);
   std::map<std::pair<int, int>, int> seen;             // (dz², |o|²) → a class of the same angle θ
   std::vector<ld> rr((size_t)ntri * nq), ri((size_t)ntri * nq);
@@ -138,10 +136,11 @@ std::shared_ptr<const RotHost> build(int p, const HostOperators& op) {
     int a2 = oz * oz, b2 = ox * ox + oy * oy + oz * oz;
     for (int g = 2; g <= a2 || (a2 == 0 && g <= b2); ++g)
       while (a2 % g == 0 && b2 % g == 0 && b2 > 1) { a2 /= g; b2 /= g; }
-    double* D = &H->d[(size_t)c * R.nd];
+    const size_t nd = (size_t)32 * R.nd;
+    double* D = &H->d[c * nd];
     const auto it = seen.find({a2, b2});
     if (it != seen.end()) {
-      std::copy(&H->d[(size_t)it->second * R.nd], &H->d[(size_t)it->second * R.nd] + R.nd, D);
+      std::copy(&H->d[it->second * nd], &H->d[it->second * nd] + nd, D);
       continue;
     }
     seen[{a2, b2}] = c;
@@ -164,7 +163,7 @@ std::shared_ptr<const RotHost> build(int p, const HostOperators& op) {
             const ld* v = bas + (size_t)(l * (l + 1) / 2 + k) * nq;
             ld sum = 0;
             for (int q = 0; q < nq; ++q) sum += u[q] * v[q];
-            D[R.re_col(l, k) + (part ? rot_pad(l + 1) + j - 1 : j)] = (double)sum;
+            D[R.rot_at(l, part, j, k)] = (double)sum;
           }
       }
   }
@@ -177,6 +176,15 @@ std::shared_ptr<const RotHost> build(int p, const HostOperators& op) {
       H->csf[((size_t)f * (p + 1) + m) * 2 + 1] = (double)(sg * std::sin(m * phi));
     }
   }
+  H->csk.assign((size_t)NCH * 2 * (p + 1), 0.0);
+  for (int k = 0; k < NCH; ++k) {
+    const ld phi = std::atan2((ld)(k >> 1 & 1) - 0.5L, (ld)(k & 1) - 0.5L);
+    for (int m = 0; m <= p; ++m) {
+      const ld sg = !(k >> 2) && (m & 1) ? -1 : 1;
+      H->csk[((size_t)k * (p + 1) + m) * 2] = (double)(sg * std::cos(m * phi));
+      H->csk[((size_t)k * (p + 1) + m) * 2 + 1] = (double)(sg * std::sin(m * phi));
+    }
+  }
   return H;
 }
 
@@ -186,7 +194,7 @@ void gauss_legendre(int n, std::vector<double>& t, std::vector<double>& w) {
   legendre_rule<double>(n, t, w, M_PI, 1e-16);
 }
 
-// built once per order in the process (at most PMAX of them, 2 MB at the largest order) and
+// built once per order in the process (at most PMAX of them, 2.5 MB at the largest order) and
 // shared by every cache; the classes and their representatives are the same for every order
 std::shared_ptr<const RotHost> rotation_tables(int p, const HostOperators& op) {
   static std::mutex mu;

@@ -4,10 +4,10 @@
 // (Ψ̂ = Ψ_c/w in the box's own coordinates), nexp·LD apart; they use the scalar operators of
 // SphericalHarmonics with the couplings of the reference:
 //   P2M  block k: charges f_k; block 4: charges ŷ·f (ŷ = (y − c)/w)        (harmonics_stokes.jl:322-328)
-//   M2M  Ψ̂_P = ½ Ψ̂_C + δ̂·Φ_C folded into the stacked children before the product (:136-158)
-//   M2L  Ψ̂_B += T(Ψ̂_A + o·Φ_A), o the far offset (linear in the source: the gather of the fourth
-//        launch of the class-wise M2L forms it, m2l_f64.cu)                 (:77-97)
-//   L2L  children blocks 1–3 = L2L·P_a; block 4 = 2·L2L·P₄ − 2 δ̂·(L2L·P_Φ) (:159-183)
+//   M2M  Ψ̂_P = Σ M2M(½ Ψ̂_C + δ̂·Φ_C), δ̂ = (c_C − c_P)/w_P ∈ {±¼}³          (:136-158)
+//   M2L  Ψ̂_B += T(Ψ̂_A + o·Φ_A), o the far offset                             (:77-97)
+//   L2L  Ψ̂_C += L2L(2Ψ̂_P − 2 δ̂·Φ_P)                                          (:159-183)
+//        (each is linear in the source: the translations' gather forms it, m2l_rot.cu)
 //   L2P  u = ½[Φ − x̂·∇̂Φ + ∇̂Ψ̂] from the values and scaled gradients of the four blocks (:283-287)
 //   near c(f/r + d(d·f)/r³), c = 1/(8π), self excluded by index (src/kernels.jl:253-272)
 // Stresslets (f, ν) and doublets g (src/sources.jl:203-281) enter as dipole densities
@@ -26,9 +26,6 @@ constexpr double KSTOKES = 0.039788735772973833942;   // 1/(8π)
 constexpr int SW = 4;                                  // warps per block of the evaluation kernels
 
 inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t); }
-
-// δ̂ of child slot j along d: (c_child − c_parent)/w_parent ∈ {±1/4} (bit d of j = coordinate d)
-__device__ __forceinline__ double dhat(int j, int d) { return (((j >> d) & 1) ? 0.25 : -0.25); }
 
 // points and densities in tree order (perm: sorted position → original index), weighted: the
 // Stokeslets into f3 (zeros when absent), the stresslet strengths, stressvecs and doublets into
@@ -94,35 +91,6 @@ __global__ void k_stokes_q4(const int* __restrict__ nodes, int nn, const int4* _
       }
     }
   }
-}
-
-// M2M input of block a for the ng sibling groups of children starting at c0: the eight
-// children's block a stacked (8·LD per group); block 4 with ½Ψ̂ + δ̂·Φ
-__global__ void k_stokes_m2m_in(const double* __restrict__ M, int c0, int ng, int LD, int a, double* __restrict__ X) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (int64_t)ng * 8 * LD) return;
-  const int i = (int)(e % LD), j = (int)((e / LD) % 8), g = (int)(e / (8 * LD));
-  const double* ch = M + (int64_t)(c0 + 8 * g + j) * 4 * LD;
-  double v;
-  if (a < 3) v = ch[(int64_t)a * LD + i];
-  else v = 0.5 * ch[3 * (int64_t)LD + i] + dhat(j, 0) * ch[i] + dhat(j, 1) * ch[LD + i] + dhat(j, 2) * ch[2 * (int64_t)LD + i];
-  X[e] = v;
-}
-
-// L2L output: R_a = L2L·P_a (8·LD per group, a = 0..3) added to the children's partial locals,
-// block 4 as 2·R₄ − 2 δ̂·(R₁, R₂, R₃)
-__global__ void k_stokes_l2l_out(double* __restrict__ Pl, const double* __restrict__ R, int c0, int ng, int LD, int NP) {
-  const int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  const int64_t per = (int64_t)ng * 8 * LD;
-  if (e >= per) return;
-  const int i = (int)(e % LD), j = (int)((e / LD) % 8), g = (int)(e / (8 * LD));
-  if (i >= NP) return;
-  double* ch = Pl + (int64_t)(c0 + 8 * g + j) * 4 * LD;
-  const double r1 = R[e], r2 = R[per + e], r3 = R[2 * per + e], r4 = R[3 * per + e];
-  ch[i] += r1;
-  ch[LD + i] += r2;
-  ch[2 * (int64_t)LD + i] += r3;
-  ch[3 * (int64_t)LD + i] += 2.0 * r4 - 2.0 * (dhat(j, 0) * r1 + dhat(j, 1) * r2 + dhat(j, 2) * r3);
 }
 
 // the far field at the targets of one leaf: u = ½[Φ − x̂·∇̂Φ + ∇̂Ψ̂] from the leaf's four local blocks
@@ -474,32 +442,10 @@ void stokes_build(State& S, const double* xyz_dev, const StokesDensities& d) {
     M4[a] = S.M.p + (int64_t)a * LD;
   }
   p2m_blocks(S, 4, q4, d4, M4, pitch);
-  // M2M, level by level: the stacked children of each block (Ψ̂ with the coupling), one product each
-  for (int l = P.L - 2; l >= 2; --l) {
-    const int c0 = P.level_start[l + 1], ng = P.level_groups[l + 1];
-    if (ng == 0) continue;
-    DBuf<double> X((size_t)ng * NCH * LD);
-    for (int a = 0; a < 4; ++a) {
-      k_stokes_m2m_in<<<nblk((int64_t)ng * NCH * LD), 256, 0, s>>>(S.M.p, c0, ng, LD, a, X.p);
-      FMMB_LAUNCH_CHECK();
-      ColMap bm{X.p, nullptr, 0, NCH}, cm{S.M.p + (int64_t)a * LD, P.group_parent[l + 1].p, 0, 0, pitch};
-      gemm_expansions(LD, NCH * LD, P.lv_m2m[l], bm, cm, ng, LD, C.np, 0, P.ctx->num_sms, s);
-    }
-  }
-  // M2L of every block (the Ψ̂ launch with the coupling), then L2L level by level
+  // M2M, level by level, then the M2L of every block and L2L, each with the Ψ̂ coupling
+  m2m_sweep(S);
   m2l_stage(S);
-  for (int l = 3; l < P.L; ++l) {
-    const int c0 = P.level_start[l], ng = P.level_groups[l];
-    if (ng == 0) continue;
-    const int64_t per = (int64_t)ng * NCH * LD;
-    DBuf<double> R(4 * per);
-    for (int a = 0; a < 4; ++a) {
-      ColMap bm{S.Pl.p + (int64_t)a * LD, P.group_parent[l].p, 0, 0, pitch}, cm{R.p + a * per, nullptr, 0, NCH};
-      gemm_expansions(NCH * LD, LD, P.lv_l2l[l - 1], bm, cm, ng, LD, C.np, 0, P.ctx->num_sms, s);
-    }
-    k_stokes_l2l_out<<<nblk(per), 256, 0, s>>>(S.Pl.p, R.p, c0, ng, LD, C.np);
-    FMMB_LAUNCH_CHECK();
-  }
+  l2l_sweep(S);
   S.built = true;
 }
 

@@ -27,3 +27,21 @@ def test_rotated_m2l_matches_dense(oracle, fmmb, p):
         f = fmmb.FMM(fmmb.SphericalHarmonics(fmmb.Laplace3D(), p=p), pts, ppl=ppl, bbox=BOX)
         u, g = fmmb.evaluate_at_sources_both(f, fmmb.build_expansions(f, pts, tau))
         assert mrd(u, ou) < 1e-12 and mrd(g, og) < 1e-11, (name, mrd(u, ou), mrd(g, og))
+
+
+def test_order_16_same_in_a_large_launch(fmmb):
+    """At p = 16 a launch of a million pairs or more takes another shape (two groups of warps, chunks of
+    24 pairs). A pair's product and the order of a target's sums depend on neither: a batch of eight
+    instances, large, equals each instance's own plan, small, bit by bit."""
+    rng = np.random.default_rng(16)
+    m = fmmb.SphericalHarmonics(fmmb.Laplace3D(), p=16)
+    sets = [DISTRIBUTIONS3["uniform"](rng, 6000) for _ in range(8)]
+    tau = [rng.standard_normal(6000) for _ in sets]
+    batch = fmmb.BatchFMM(m, sets, ppl=4, bbox=BOX)
+    cache = fmmb.OperatorCache(m)
+    alone = [fmmb.FMM(m, s, ppl=4, bbox=BOX, cache=cache) for s in sets]
+    assert max(f.npairs for f in alone) < 1000000 <= batch.npairs
+    u, g = fmmb.evaluate_at_sources_both(batch, fmmb.build_expansions(batch, batch.sources, batch.concat(tau)))
+    for i, f in enumerate(alone):
+        a, b = fmmb.evaluate_at_sources_both(f, fmmb.build_expansions(f, sets[i], tau[i]))
+        assert np.array_equal(batch.split(u)[i], a) and np.array_equal(batch.split(g)[i], b)
