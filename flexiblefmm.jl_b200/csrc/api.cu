@@ -687,7 +687,6 @@ int fmmb_state_create(fmmb_plan* plan, int precision, fmmb_state** out) {
       std::lock_guard<std::mutex> lk(P.cache->mu);
       prepare_rotations(P);
     }
-    apply_tuned_state(S);                         // the launch shapes tuned for states of this kind
     FMMB_CUDA(cudaStreamSynchronize(s));
     h->parent = plan;
     std::lock_guard<std::mutex> lk(g_handles);

@@ -3,26 +3,23 @@
 //   k_l2p   the far field: L2P of the leaf's local expansion (harmonics.jl:447-486), one warp
 //           per leaf group with the local staged in shared memory, lanes over the targets; FP64 on
 //           the plain path, FP32 on the mixed path (tolerances ≥ 1e-8); writes the outputs
-//   k_near  the near field: the sources of the 27 colleagues, flattened into batches of 32 that
-//           each warp stages once in shared memory while the next batch's loads are in flight;
-//           lanes over the targets; adds to the outputs. The self term is skipped by index
-//           (evaluate_at_sources, src/evaluate.jl:1-10), checked only in the batches that hold
-//           the leaf's own points.
+//   k_near  the near field (near.cuh): the sources of the 27 colleagues, flattened into batches of 32
+//           that the warps of a leaf's team stage in shared memory, lanes over the targets; adds to
+//           the outputs. The self term is skipped by index (evaluate_at_sources,
+//           src/evaluate.jl:1-10), checked only in the batches that hold the leaf's own points.
 // Two precisions of the near field:
 //   double  the plain path: absolute coordinates, the reference's FMA square norm
-//           (src/kernels.jl:20-24) and its summation order (colleagues in order, points in order)
+//           (src/kernels.jl:20-24)
 //   float   the mixed path: coordinates relative to the target leaf's centre, converted from FP64
 //           when staged (the FP32 differences carry an absolute error of ~2⁻²⁴·w instead of
 //           2⁻²⁴·|x|, so close pairs keep their accuracy); two sources per packed f32x2
 //           instruction; each batch summed in FP32, the batch sums accumulated in FP64
 // Splitting the two keeps the near-field loop at a low register count (high occupancy); the
 // outputs are u then u + KC·near, the same arithmetic as one fused pass.
-#include "passes.cuh"
+#include "near.cuh"
 
 namespace fmmb {
 namespace {
-
-constexpr int NEAR_WARPS = 4;
 
 // The leaf's local expansion prepared for L2P (harmonics.jl:447-486): per (m, n), m-major, eight
 // values — the potential's coefficient pair and the three gradient components' pairs (each from
@@ -170,80 +167,6 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
   return r;
 }
 
-template <typename R>
-struct NearWarp {
-  R4<R> stg[2][32];   // double-buffered batch of staged sources
-  int lo[32];         // first point of each colleague (27 used)
-  int pre[32];        // flat index of each colleague's first point (total for the unused slots)
-};
-
-// the sources of batch b (flat indices 32b + lane) from global memory, in FP64
-template <typename R>
-__device__ __forceinline__ void load_batch(const NearWarp<R>& sw, int b, int lane, int S, const double* __restrict__ xs,
-                                           const double* __restrict__ ys, const double* __restrict__ zs,
-                                           const double* __restrict__ q, double& x, double& y, double& z, double& w) {
-  const int f = 32 * b + lane;
-  x = y = z = w = 0.0;
-  if (f < S) {
-    int idx = 0;   // the last colleague whose flat start is ≤ f
-#pragma unroll
-    for (int step = 16; step; step >>= 1)
-      if (sw.pre[idx + step] <= f) idx += step;
-    const int j = sw.lo[idx] + (f - sw.pre[idx]);
-    x = xs[j];
-    y = ys[j];
-    z = zs[j];
-    w = q[j];
-  }
-}
-
-// one batch of m staged sources against this lane's target; CHECK skips flat index `is`.
-// YK (FP64): the Yukawa pair e^{−κr}/r and its radial derivative −e^{−κr}(1 + κr)/r²
-// (src/kernels.jl:235-242)
-// KIND 2 (FP64): the Laplace2D pair c·log r², c = −1/(4π), as KC·(−τ log r²) and gradient
-// −KC·(2τ/r²)·d (src/kernels.jl:58-66; the points share z, so r² is the planar distance)
-template <typename R, bool CHECK, int YK = 0>
-__device__ __forceinline__ void near_batch(const R4<R>* __restrict__ stg, int m, int is, R fx, R fy, R fz, R& bp, R& bx,
-                                           R& by, R& bz, double kappa = 0) {
-  auto body = [&](int i) {
-    const R4<R> sv = stg[i];
-    const R dx = fx - sv.x, dy = fy - sv.y, dz = fz - sv.z;
-    R r2, ir;
-    if constexpr (sizeof(R) == 8) {
-      r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-      ir = rsqrt(r2);
-    } else {
-      r2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-      ir = rsqrt_ftz(r2);
-    }
-    if (CHECK && i == is) ir = R(0);
-    R qir, qir3;
-    if constexpr (YK == 2) {
-      const bool self = CHECK && i == is;
-      qir = self ? R(0) : -sv.w * log(r2);
-      qir3 = self ? R(0) : 2 * sv.w / r2;
-    } else if constexpr (YK == 1) {
-      const double r = r2 * ir, e = exp(-kappa * r);
-      qir = sv.w * e * ir;
-      qir3 = qir * (1 + kappa * r) * ir * ir;
-    } else {
-      qir = sv.w * ir;
-      qir3 = qir * ir * ir;
-    }
-    bp += qir;
-    bx = fma(qir3, dx, bx);
-    by = fma(qir3, dy, by);
-    bz = fma(qir3, dz, bz);
-  };
-  if (m == 32) {
-#pragma unroll 8
-    for (int i = 0; i < 32; ++i) body(i);
-  } else {
-#pragma unroll 4
-    for (int i = 0; i < m; ++i) body(i);
-  }
-}
-
 // packed FP32 pairs (the f32x2 instructions of sm_100: two lanes of arithmetic per instruction)
 __device__ __forceinline__ uint64_t pk2(float a, float b) {
   uint64_t r;
@@ -266,169 +189,156 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
   return d;
 }
-__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
 
-// The FP32 batch with two sources per instruction: the batch staged as 16 source pairs
-// {x₀ x₁ y₀ y₁}{z₀ z₁ w₀ w₁}; each pair's arithmetic in packed f32x2 (the same operations and
-// per-element rounding as near_batch), the two running sums of every quantity added at the end;
-// an odd last source takes the scalar body. CHECK skips flat index `is`.
-template <bool CHECK>
-__device__ __forceinline__ void near_batch_f32x2(const float4* __restrict__ pr, int m, int is, float fx, float fy,
-                                                 float fz, float& bp, float& bx, float& by, float& bz) {
-  const uint64_t fx2 = pk2(fx, fx), fy2 = pk2(fy, fy), fz2 = pk2(fz, fz);
-  uint64_t p2 = pk2(0.f, 0.f), x2 = p2, y2 = p2, z2 = p2;
-  const int np = m >> 1;
-  auto body = [&](int k) {
-    const float4 a = pr[2 * k], b = pr[2 * k + 1];
-    const uint64_t dx = sub2(fx2, pk2(a.x, a.y)), dy = sub2(fy2, pk2(a.z, a.w)), dz = sub2(fz2, pk2(b.x, b.y));
-    const uint64_t r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
-    float ra, rb;
-    upk2(r2, ra, rb);
-    float ia = rsqrt_ftz(ra), ib = rsqrt_ftz(rb);
-    if (CHECK && 2 * k == is) ia = 0.f;
-    if (CHECK && 2 * k + 1 == is) ib = 0.f;
-    const uint64_t ir = pk2(ia, ib);
-    const uint64_t qir = mul2(pk2(b.z, b.w), ir);
-    const uint64_t qir3 = mul2(mul2(qir, ir), ir);
-    p2 = add2(p2, qir);
-    x2 = fma2(qir3, dx, x2);
-    y2 = fma2(qir3, dy, y2);
-    z2 = fma2(qir3, dz, z2);
+// The near field of charges (near.cuh). KERNEL 0: Laplace3D; 1 (FP64): the Yukawa pair e^{−κr}/r and
+// its radial derivative −e^{−κr}(1 + κr)/r² (src/kernels.jl:235-242); 2 (FP64): the Laplace2D pair
+// c·log r², c = −1/(4π), as KC·(−τ log r²) and gradient −KC·(2τ/r²)·d (src/kernels.jl:58-66; the
+// points share z, so r² is the planar distance). GRAD: the gradient's sums too.
+template <typename R, int KERNEL, bool GRAD>
+struct ChargesNear {
+  using Real = R;
+  static constexpr bool REL = sizeof(R) == 4;   // the mixed path works relative to the leaf's centre
+  static constexpr int NA = GRAD ? 4 : 1, CH = 2, MINB = KERNEL == 2 ? 4 : 5;
+  struct Args {
+    const double *xs, *ys, *zs, *q;
+    double kappa;
+    int outputs, first;       // first: the far field comes after (and adds to) the outputs
+    double *pot, *grad;
   };
-  if (np == 16) {
+  struct Src { double x, y, z, w; };
+  struct Stage { R4<R> s[32]; };
+  static __device__ __forceinline__ void load(const Args& a, int j, Src& v) { v = Src{a.xs[j], a.ys[j], a.zs[j], a.q[j]}; }
+  static __device__ __forceinline__ void stage(Stage& st, int lane, const Src& v, double cx, double cy, double cz) {
+    if constexpr (sizeof(R) == 4) {
+      // source pairs {x₀ x₁ y₀ y₁}{z₀ z₁ w₀ w₁}: lane l into pair l/2, slot l%2
+      float* f = reinterpret_cast<float*>(st.s) + 8 * (lane >> 1) + (lane & 1);
+      f[0] = (float)(v.x - cx);
+      f[2] = (float)(v.y - cy);
+      f[4] = (float)(v.z - cz);
+      f[6] = (float)v.w;
+    } else {
+      st.s[lane] = R4<R>{(R)v.x, (R)v.y, (R)v.z, (R)v.w};
+    }
+  }
+  // m staged sources against this lane's target; CHECK skips source `is`; the lane's part of f of them
+  template <bool CHECK>
+  static __device__ __forceinline__ void batch(const Args& pa, const Stage& st, int m, int is, int part, int f, const R (&t)[3],
+                                               double (&acc)[NA]) {
+    if constexpr (sizeof(R) == 4) batch_f32x2<CHECK>(st, m, is, part, f, t, acc);
+    else batch_f64<CHECK>(pa, st, m, is, part, f, t, acc);
+  }
+  // the plain path sums straight into the FP64 totals
+  template <bool CHECK>
+  static __device__ __forceinline__ void batch_f64(const Args& pa, const Stage& st, int m, int is, int part, int f,
+                                                   const double (&t)[3], double (&acc)[NA]) {
+    auto body = [&](int i) {
+      const R4<R> sv = st.s[i];
+      const double dx = t[0] - sv.x, dy = t[1] - sv.y, dz = t[2] - sv.z;
+      const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+      // the potential's sums in explicit FMAs: the same bits with and without the gradient's
+      double qir3 = 0;
+      if constexpr (KERNEL == 2) {
+        const bool self = CHECK && i == is;
+        acc[0] = fma(-sv.w, self ? 0.0 : log(r2), acc[0]);
+        if (GRAD) qir3 = self ? 0.0 : 2 * sv.w / r2;
+      } else {
+        double ir = rsqrt_h(r2), w = sv.w;
+        if (CHECK && i == is) ir = 0.0;
+        if constexpr (KERNEL == 1) {
+          const double kr = __dmul_rn(pa.kappa, __dmul_rn(r2, ir));
+          w = __dmul_rn(w, exp(-kr));
+          if (GRAD) qir3 = w * (1 + kr) * ir * ir * ir;
+        } else {
+          if (GRAD) qir3 = w * ir * ir * ir;
+        }
+        acc[0] = fma(w, ir, acc[0]);
+      }
+      if constexpr (GRAD) {
+        acc[1] = fma(qir3, dx, acc[1]);
+        acc[2] = fma(qir3, dy, acc[2]);
+        acc[3] = fma(qir3, dz, acc[3]);
+      }
+    };
+    if (m == 32 && f == 1) {
 #pragma unroll 8
-    for (int k = 0; k < 16; ++k) body(k);
-  } else {
+      for (int i = 0; i < 32; ++i) body(i);
+    } else {
+#pragma unroll 4
+      for (int i = part; i < m; i += f) body(i);
+    }
+  }
+  // two sources per instruction: each pair's arithmetic in packed f32x2, the two running sums of
+  // every quantity added at the end and the batch's sums accumulated in FP64; an odd last source
+  // takes a scalar body
+  template <bool CHECK>
+  static __device__ __forceinline__ void batch_f32x2(const Stage& st, int m, int is, int part, int f, const R (&t)[3],
+                                                     double (&acc)[NA]) {
+    const float4* pr = reinterpret_cast<const float4*>(st.s);
+    const float fx = t[0], fy = t[1], fz = t[2];
+    const uint64_t fx2 = pk2(fx, fx), fy2 = pk2(fy, fy), fz2 = pk2(fz, fz);
+    uint64_t p2 = pk2(0.f, 0.f), x2 = p2, y2 = p2, z2 = p2;
+    const int np = m >> 1;
+    auto body = [&](int k) {
+      const float4 a = pr[2 * k], b = pr[2 * k + 1];
+      const uint64_t dx = sub2(fx2, pk2(a.x, a.y)), dy = sub2(fy2, pk2(a.z, a.w)), dz = sub2(fz2, pk2(b.x, b.y));
+      const uint64_t r2 = fma2(dz, dz, fma2(dy, dy, mul2(dx, dx)));
+      float ra, rb;
+      upk2(r2, ra, rb);
+      float ia = rsqrt_ftz(ra), ib = rsqrt_ftz(rb);
+      if (CHECK && 2 * k == is) ia = 0.f;
+      if (CHECK && 2 * k + 1 == is) ib = 0.f;
+      const uint64_t ir = pk2(ia, ib);
+      const uint64_t w = pk2(b.z, b.w);
+      p2 = fma2(w, ir, p2);                        // explicit: the same bits with and without the gradient
+      if constexpr (GRAD) {
+        const uint64_t qir3 = mul2(mul2(mul2(w, ir), ir), ir);
+        x2 = fma2(qir3, dx, x2);
+        y2 = fma2(qir3, dy, y2);
+        z2 = fma2(qir3, dz, z2);
+      }
+    };
+    if (np == 16 && f == 1) {
+#pragma unroll 8
+      for (int k = 0; k < 16; ++k) body(k);
+    } else {
 #pragma unroll 2
-    for (int k = 0; k < np; ++k) body(k);
+      for (int k = part; k < np; k += f) body(k);
+    }
+    float bp, bx, by, bz, hi;
+    upk2(p2, bp, hi); bp += hi;
+    if constexpr (GRAD) {
+      upk2(x2, bx, hi); bx += hi;
+      upk2(y2, by, hi); by += hi;
+      upk2(z2, bz, hi); bz += hi;
+    }
+    if ((m & 1) && part == 0) {                    // the odd last source
+      const float* g = reinterpret_cast<const float*>(pr + 2 * np);
+      const float dx = fx - g[0], dy = fy - g[2], dz = fz - g[4];
+      float ir = rsqrt_ftz(fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
+      if (CHECK && m - 1 == is) ir = 0.f;
+      bp = fmaf(g[6], ir, bp);
+      if constexpr (GRAD) {
+        const float qir3 = g[6] * ir * ir * ir;
+        bx = fmaf(qir3, dx, bx);
+        by = fmaf(qir3, dy, by);
+        bz = fmaf(qir3, dz, bz);
+      }
+    }
+    acc[0] += bp;
+    if constexpr (GRAD) { acc[1] += bx; acc[2] += by; acc[3] += bz; }
   }
-  float a0, a1;
-  upk2(p2, a0, a1); bp += a0 + a1;
-  upk2(x2, a0, a1); bx += a0 + a1;
-  upk2(y2, a0, a1); by += a0 + a1;
-  upk2(z2, a0, a1); bz += a0 + a1;
-  if (m & 1) {                                   // the odd last source
-    const float* f = reinterpret_cast<const float*>(pr + 2 * np);
-    const float dx = fx - f[0], dy = fy - f[2], dz = fz - f[4];
-    float ir = rsqrt_ftz(fmaf(dz, dz, fmaf(dy, dy, dx * dx)));
-    if (CHECK && m - 1 == is) ir = 0.f;
-    const float qir = f[6] * ir, qir3 = qir * ir * ir;
-    bp += qir;
-    bx = fmaf(qir3, dx, bx);
-    by = fmaf(qir3, dy, by);
-    bz = fmaf(qir3, dz, bz);
-  }
-}
-
-// W warps (leaf groups) per CTA: 4 or 8, chosen per state by the tuner (tune.cu)
-template <typename R, bool SELF, int YK, int W>
-__global__ void __launch_bounds__(W * 32, W == 4 ? 5 : 2) k_near(const int* __restrict__ gnode, const int* __restrict__ gstart,
-                                                         const int* __restrict__ gcount, int ngroups,
-                                                         const double* __restrict__ tx, const double* __restrict__ ty,
-                                                         const double* __restrict__ tz, const int* __restrict__ tout,
-                                                         const double* __restrict__ xs, const double* __restrict__ ys,
-                                                         const double* __restrict__ zs, const double* __restrict__ q,
-                                                         const int4* __restrict__ cell, const int* __restrict__ plo,
-                                                         const int* __restrict__ phi, const int* __restrict__ col,
-                                                         Geometry geo, int outputs, double* __restrict__ pot,
-                                                         double* __restrict__ grad, double kappa, int first) {
-  constexpr bool REL = sizeof(R) == 4;   // the mixed path works relative to the leaf's centre
-  __shared__ NearWarp<R> sws[W];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int grp = blockIdx.x * W + warp;
-  if (grp >= ngroups) return;                      // the whole warp
-  NearWarp<R>& sw = sws[warp];
-  const int leaf = gnode[grp];
-  double cx = 0, cy = 0, cz = 0;
-  if (REL) {
-    const int4 c = cell[leaf];
-    const Geometry gn = geo.at(leaf);
-    const double w = ldexp(geo.W0, -c.w);
-    cx = gn.center(0, c.x, w);
-    cy = gn.center(1, c.y, w);
-    cz = gn.center(2, c.z, w);
-  }
-  // the colleagues' point ranges, flattened in colleague order
-  const int cn = lane < NCOL ? col[(int64_t)leaf * NCOL + lane] : -1;
-  int lo = 0, len = 0;
-  if (cn >= 0) {
-    lo = plo[cn];
-    len = max(0, phi[cn] - lo + 1);
-  }
-  int incl = len;
+  static __device__ __forceinline__ void write(const Args& a, int o, const double (&acc)[NA]) {
+    // a product and a sum, never one FMA: the near field may come before or after the far field
+    if (a.outputs & FMMB_OUTPUT_POTENTIAL) a.pot[o] = __dadd_rn(a.first ? 0.0 : a.pot[o], __dmul_rn(KC, acc[0]));
+    if constexpr (GRAD) {
+      if (a.outputs & FMMB_OUTPUT_GRADIENT) {
+        double* g = a.grad + 3 * (int64_t)o;
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  const int S = __shfl_sync(0xffffffffu, incl, 31);
-  sw.lo[lane] = lo;
-  sw.pre[lane] = incl - len;
-  // the leaf's own slot: its points are the self terms
-  const unsigned selfm = __ballot_sync(0xffffffffu, cn == leaf);
-  const int slot = selfm ? __ffs(selfm) - 1 : 0;
-  const int pself = selfm ? __shfl_sync(0xffffffffu, incl - len, slot) : -1;
-  const int loself = __shfl_sync(0xffffffffu, lo, slot), lenself = selfm ? __shfl_sync(0xffffffffu, len, slot) : 0;
-  __syncwarp();
-  const int t0 = gstart[grp], nt = gcount[grp];
-  for (int base = 0; base < nt; base += 32) {
-    const int k = t0 + base + lane;
-    const bool act = base + lane < nt;
-    const double x = act ? tx[k] : cx, y = act ? ty[k] : cy, z = act ? tz[k] : cz;
-    const R fx = (R)(x - cx), fy = (R)(y - cy), fz = (R)(z - cz);
-    const int fself = SELF && act && selfm ? pself + (k - loself) : -1;
-    double np = 0, nx = 0, ny = 0, nz = 0;
-    double sx, sy, sz, sq;
-    load_batch(sw, 0, lane, S, xs, ys, zs, q, sx, sy, sz, sq);
-    for (int b = 0; 32 * b < S; ++b) {
-      R4<R>* stg = sw.stg[b & 1];
-      if constexpr (sizeof(R) == 4) {
-        // the FP32 path stages source pairs: lane l into pair l/2, slot l%2
-        float* f = reinterpret_cast<float*>(stg) + 8 * (lane >> 1) + (lane & 1);
-        f[0] = (float)(sx - cx);
-        f[2] = (float)(sy - cy);
-        f[4] = (float)(sz - cz);
-        f[6] = (float)sq;
-      } else {
-        stg[lane] = R4<R>{(R)(sx - cx), (R)(sy - cy), (R)(sz - cz), (R)sq};
-      }
-      __syncwarp();
-      if (32 * (b + 1) < S) load_batch(sw, b + 1, lane, S, xs, ys, zs, q, sx, sy, sz, sq);
-      const int m = min(32, S - 32 * b);
-      const bool chk = SELF && selfm && 32 * b < pself + lenself && 32 * b + 32 > pself;   // uniform
-      if constexpr (sizeof(R) == 8) {
-        // the plain path sums straight into the FP64 totals, in the reference's order
-        if (chk) near_batch<R, true, YK>(stg, m, fself - 32 * b, fx, fy, fz, np, nx, ny, nz, kappa);
-        else near_batch<R, false, YK>(stg, m, 0, fx, fy, fz, np, nx, ny, nz, kappa);
-      } else {
-        float bp = 0, bx = 0, by = 0, bz = 0;
-        const float4* pr = reinterpret_cast<const float4*>(stg);
-        if (chk) near_batch_f32x2<true>(pr, m, fself - 32 * b, fx, fy, fz, bp, bx, by, bz);
-        else near_batch_f32x2<false>(pr, m, 0, fx, fy, fz, bp, bx, by, bz);
-        np += bp;
-        nx += bx;
-        ny += by;
-        nz += bz;
+        for (int d = 0; d < 3; ++d) g[d] = __dadd_rn(a.first ? 0.0 : g[d], -__dmul_rn(KC, acc[1 + d]));
       }
     }
-    if (act) {
-      const int o = tout[k];
-      // first: the far field comes after (and adds to) these
-      if (outputs & FMMB_OUTPUT_POTENTIAL) pot[o] = (first ? 0.0 : pot[o]) + KC * np;
-      if (outputs & FMMB_OUTPUT_GRADIENT) {
-        const int64_t o3 = 3 * (int64_t)o;
-        grad[o3] = (first ? 0.0 : grad[o3]) - KC * nx;
-        grad[o3 + 1] = (first ? 0.0 : grad[o3 + 1]) - KC * ny;
-        grad[o3 + 2] = (first ? 0.0 : grad[o3 + 2]) - KC * nz;
-      }
-    }
-    __syncwarp();   // the staging buffers are reused by the next group of targets
   }
-}
+};
 
 // The kernel-independent far field (l2t, src/operators/ki_common.jl:293-327): at each target
 // Σ_k G(x − y_k) L_k over the leaf's large surface y_k = c + w·ŷ_k (ŷ at width 1), times w (the
@@ -570,111 +480,63 @@ __global__ void __launch_bounds__(128) k_kic_l2t(const int* __restrict__ gnode, 
   }
 }
 
-// The near field of charges and dipoles (source_field / target_field of src/sources.jl:137-155 with
-// Laplace3D): per source q/r + (d·v)/r³ and the gradient −q v/r³ + d/r³ − 3 v (d·v)/r⁵, v = t − s,
-// as KC times the sums below (pot += KC·Σ, grad −= KC·Σ). Same flattening of the colleagues'
-// ranges as k_near, one batch of 32 staged sources (positions and moments) at a time; R as there
-// (FP32 relative to the leaf's centre with FP64 batch sums, or FP64).
-template <typename R, bool SELF>
-__global__ void __launch_bounds__(NEAR_WARPS * 32) k_near_dip(const int* __restrict__ gnode, const int* __restrict__ gstart,
-                                                             const int* __restrict__ gcount, int ngroups,
-                                                             const double* __restrict__ tx, const double* __restrict__ ty,
-                                                             const double* __restrict__ tz, const int* __restrict__ tout,
-                                                             const double* __restrict__ xs, const double* __restrict__ ys,
-                                                             const double* __restrict__ zs, const double* __restrict__ q,
-                                                             const double* __restrict__ d3, int64_t npts,
-                                                             const int4* __restrict__ cell, const int* __restrict__ plo,
-                                                             const int* __restrict__ phi, const int* __restrict__ col,
-                                                             Geometry geo, int outputs, double* __restrict__ pot,
-                                                             double* __restrict__ grad) {
-  constexpr bool REL = sizeof(R) == 4;
-  __shared__ R4<R> sp[NEAR_WARPS][32], sd[NEAR_WARPS][32];
-  __shared__ int slo[NEAR_WARPS][32], spre[NEAR_WARPS][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int grp = blockIdx.x * NEAR_WARPS + warp;
-  if (grp >= ngroups) return;
-  const int leaf = gnode[grp];
-  double cx = 0, cy = 0, cz = 0;
-  if (REL) {
-    const int4 c = cell[leaf];
-    const Geometry gn = geo.at(leaf);
-    const double w = ldexp(geo.W0, -c.w);
-    cx = gn.center(0, c.x, w);
-    cy = gn.center(1, c.y, w);
-    cz = gn.center(2, c.z, w);
+// The near field of charges and dipoles (near.cuh; source_field / target_field of
+// src/sources.jl:137-155 with Laplace3D): per source q/r + (d·v)/r³ and the gradient
+// −q v/r³ + d/r³ − 3 v (d·v)/r⁵, v = t − s, as KC times the sums below (pot += KC·Σ, grad −= KC·Σ);
+// coincident points contribute nothing. R = float: relative to the leaf's centre, batches summed in
+// FP32 and their sums in FP64.
+template <typename R>
+struct DipolesNear {
+  using Real = R;
+  static constexpr bool REL = sizeof(R) == 4;
+  static constexpr int NA = 4, CH = 2, MINB = 4;
+  struct Args {
+    const double *xs, *ys, *zs, *q, *d3;
+    int64_t npts;
+    int outputs;
+    double *pot, *grad;
+  };
+  struct Src { double x, y, z, q, dx, dy, dz; };
+  struct Stage { R4<R> p[32], d[32]; };
+  static __device__ __forceinline__ void load(const Args& a, int j, Src& v) {
+    v = Src{a.xs[j], a.ys[j], a.zs[j], a.q[j], a.d3[j], a.d3[a.npts + j], a.d3[2 * a.npts + j]};
   }
-  const int cn = lane < NCOL ? col[(int64_t)leaf * NCOL + lane] : -1;
-  int lo = 0, len = 0;
-  if (cn >= 0) {
-    lo = plo[cn];
-    len = max(0, phi[cn] - lo + 1);
+  static __device__ __forceinline__ void stage(Stage& st, int lane, const Src& v, double cx, double cy, double cz) {
+    st.p[lane] = R4<R>{(R)(v.x - cx), (R)(v.y - cy), (R)(v.z - cz), (R)v.q};
+    st.d[lane] = R4<R>{(R)v.dx, (R)v.dy, (R)v.dz, (R)0};
   }
-  int incl = len;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  const int S = __shfl_sync(0xffffffffu, incl, 31);
-  slo[warp][lane] = lo;
-  spre[warp][lane] = incl - len;
-  __syncwarp();
-  const int t0 = gstart[grp], nt = gcount[grp];
-  for (int base = 0; base < nt; base += 32) {
-    const int k = t0 + base + lane;
-    const bool act = base + lane < nt;
-    const double x = act ? tx[k] : cx, y = act ? ty[k] : cy, z = act ? tz[k] : cz;
-    const R fx = (R)(x - cx), fy = (R)(y - cy), fz = (R)(z - cz);
-    double np = 0, nx = 0, ny = 0, nz = 0;
-    for (int b = 0; 32 * b < S; ++b) {
-      const int f = 32 * b + lane;
-      int src = -1;
-      if (f < S) {
-        int idx = 0;
-#pragma unroll
-        for (int step = 16; step; step >>= 1)
-          if (spre[warp][idx + step] <= f) idx += step;
-        src = slo[warp][idx] + (f - spre[warp][idx]);
-      }
-      __syncwarp();
-      if (src >= 0) {
-        sp[warp][lane] = R4<R>{(R)(xs[src] - cx), (R)(ys[src] - cy), (R)(zs[src] - cz), (R)q[src]};
-        sd[warp][lane] = R4<R>{(R)d3[src], (R)d3[npts + src], (R)d3[2 * npts + src], (R)0};
-      }
-      // the source index of each staged slot, for the self check
-      const int sidx = src;
-      __syncwarp();
-      const int m = min(32, S - 32 * b);
-      R bp = 0, bx = 0, by = 0, bz = 0;
-      for (int i = 0; i < m; ++i) {
-        const R4<R> sv = sp[warp][i], dv = sd[warp][i];
-        const int si = __shfl_sync(0xffffffffu, sidx, i);
-        const R vx = fx - sv.x, vy = fy - sv.y, vz = fz - sv.z;
-        const R r2 = vx * vx + vy * vy + vz * vz;
-        R ir = r2 > R(0) ? R(1) / sqrt(r2) : R(0);
-        if (SELF && act && si == k) ir = R(0);     // the target's own source: k is its tree index
-        const R ir2 = ir * ir, ir3 = ir2 * ir;
-        const R dd = dv.x * vx + dv.y * vy + dv.z * vz;
-        bp += sv.w * ir + dd * ir3;
-        const R cv = sv.w * ir3 + 3 * dd * ir3 * ir2;
-        bx += cv * vx - dv.x * ir3;
-        by += cv * vy - dv.y * ir3;
-        bz += cv * vz - dv.z * ir3;
-      }
-      np += bp; nx += bx; ny += by; nz += bz;
+  template <bool CHECK>
+  static __device__ __forceinline__ void batch(const Args&, const Stage& st, int m, int is, int part, int f, const R (&t)[3],
+                                               double (&acc)[NA]) {
+    R bp = 0, bx = 0, by = 0, bz = 0;
+#pragma unroll 2
+    for (int i = part; i < m; i += f) {
+      const R4<R> sv = st.p[i], dv = st.d[i];
+      const R vx = t[0] - sv.x, vy = t[1] - sv.y, vz = t[2] - sv.z;
+      const R r2 = vx * vx + vy * vy + vz * vz;
+      R ir;
+      if constexpr (sizeof(R) == 8) ir = r2 > 0.0 ? rsqrt_h(r2) : 0.0;
+      else ir = r2 > 0.f ? 1.f / sqrtf(r2) : 0.f;
+      if (CHECK && i == is) ir = R(0);
+      const R ir2 = ir * ir, ir3 = ir2 * ir;
+      const R dd = dv.x * vx + dv.y * vy + dv.z * vz;
+      bp += sv.w * ir + dd * ir3;
+      const R cv = sv.w * ir3 + 3 * dd * ir3 * ir2;
+      bx += cv * vx - dv.x * ir3;
+      by += cv * vy - dv.y * ir3;
+      bz += cv * vz - dv.z * ir3;
     }
-    if (act) {
-      const int o = tout[k];
-      if (outputs & FMMB_OUTPUT_POTENTIAL) pot[o] = pot[o] + KC * np;
-      if (outputs & FMMB_OUTPUT_GRADIENT) {
-        grad[3 * (int64_t)o] = grad[3 * (int64_t)o] - KC * nx;
-        grad[3 * (int64_t)o + 1] = grad[3 * (int64_t)o + 1] - KC * ny;
-        grad[3 * (int64_t)o + 2] = grad[3 * (int64_t)o + 2] - KC * nz;
-      }
-    }
-    __syncwarp();
+    acc[0] += bp; acc[1] += bx; acc[2] += by; acc[3] += bz;
   }
-}
+  static __device__ __forceinline__ void write(const Args& a, int o, const double (&acc)[NA]) {
+    if (a.outputs & FMMB_OUTPUT_POTENTIAL) a.pot[o] += KC * acc[0];
+    if (a.outputs & FMMB_OUTPUT_GRADIENT) {
+      double* g = a.grad + 3 * (int64_t)o;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) g[d] -= KC * acc[1 + d];
+    }
+  }
+};
 
 template <int P>
 void launch_l2p(State& S, const int* gnode, const int* gstart, const int* gcount, int ng, const double* tx, const double* ty,
@@ -696,21 +558,35 @@ void launch_l2p(State& S, const int* gnode, const int* gstart, const int* gcount
   FMMB_LAUNCH_CHECK();
 }
 
-template <typename R, bool SELF, int YK = 0>
+NearArgs near_args(const Plan& P, const int* gnode, const int* gstart, const int* gcount, int ng, const double* tx,
+                   const double* ty, const double* tz, const int* tout) {
+  return NearArgs{gnode, gstart, gcount, ng, tx, ty, tz, tout, P.cell.p, P.plo.p, P.phi.p, P.col.p, geometry(P)};
+}
+
+template <typename R, bool SELF, int KERNEL = 0>
 void launch_near(State& S, const int* gnode, const int* gstart, const int* gcount, int ng, const double* tx, const double* ty,
                  const double* tz, const int* tout, int outputs, double* pot, double* grad, int first = 0,
                  cudaStream_t st = nullptr) {
   Plan& P_ = *S.plan;
   const cudaStream_t s = st ? st : P_.ctx->stream;
-  if (S.near_warps == 8)
-    k_near<R, SELF, YK, 8><<<(ng + 7) / 8, 32 * 8, 0, s>>>(gnode, gstart, gcount, ng, tx, ty, tz, tout, S.xs.p, S.ys.p, S.zs.p,
-                                                          S.q.p, P_.cell.p, P_.plo.p, P_.phi.p, P_.col.p, geometry(P_),
-                                                          outputs, pot, grad, P_.cache->kappa, first);
-  else
-    k_near<R, SELF, YK, 4><<<(ng + 3) / 4, 32 * 4, 0, s>>>(gnode, gstart, gcount, ng, tx, ty, tz, tout, S.xs.p, S.ys.p, S.zs.p,
-                                                          S.q.p, P_.cell.p, P_.plo.p, P_.phi.p, P_.col.p, geometry(P_),
-                                                          outputs, pot, grad, P_.cache->kappa, first);
-  FMMB_LAUNCH_CHECK();
+  const NearArgs A = near_args(P_, gnode, gstart, gcount, ng, tx, ty, tz, tout);
+  auto go = [&](auto pol) {
+    using Pol = decltype(pol);
+    const typename Pol::Args pa{S.xs.p, S.ys.p, S.zs.p, S.q.p, P_.cache->kappa, outputs, first, pot, grad};
+    launch_near_leaves<Pol, SELF>(A, pa, P_.ctx->num_sms, s);
+  };
+  if (outputs & FMMB_OUTPUT_GRADIENT) go(ChargesNear<R, KERNEL, true>{});
+  else go(ChargesNear<R, KERNEL, false>{});
+}
+
+template <typename R, bool SELF>
+void launch_near_dip(State& S, const int* gnode, const int* gstart, const int* gcount, int ng, const double* tx,
+                     const double* ty, const double* tz, const int* tout, int outputs, double* pot, double* grad) {
+  Plan& P_ = *S.plan;
+  using Pol = DipolesNear<R>;
+  const typename Pol::Args pa{S.xs.p, S.ys.p, S.zs.p, S.q.p, S.dip.p, P_.N, outputs, pot, grad};
+  launch_near_leaves<Pol, SELF>(near_args(P_, gnode, gstart, gcount, ng, tx, ty, tz, tout), pa, P_.ctx->num_sms,
+                                P_.ctx->stream);
 }
 
 }  // namespace
@@ -751,24 +627,15 @@ void evaluate_groups(State& S, const int* gnode, const int* gstart, const int* g
   }
   const bool mixed = S.precision == FMMB_PRECISION_MIXED;
   if (S.has_dip) {
-    Plan& P_ = *S.plan;
-    const unsigned nb = (ng + NEAR_WARPS - 1) / NEAR_WARPS;
-#define FMMB_NEAR_DIP(R, SELF)                                                                                  \
-  k_near_dip<R, SELF><<<nb, 32 * NEAR_WARPS, 0, P_.ctx->stream>>>(gnode, gstart, gcount, ng, tx, ty, tz, tout, S.xs.p, \
-                                                                  S.ys.p, S.zs.p, S.q.p, S.dip.p, P_.N, P_.cell.p,     \
-                                                                  P_.plo.p, P_.phi.p, P_.col.p, geometry(P_), outputs, \
-                                                                  pot, grad)
-    if (mixed && self) FMMB_NEAR_DIP(float, true);
-    else if (mixed) FMMB_NEAR_DIP(float, false);
-    else if (self) FMMB_NEAR_DIP(double, true);
-    else FMMB_NEAR_DIP(double, false);
-#undef FMMB_NEAR_DIP
-    FMMB_LAUNCH_CHECK();
+    if (mixed && self) launch_near_dip<float, true>(S, gnode, gstart, gcount, ng, tx, ty, tz, tout, outputs, pot, grad);
+    else if (mixed) launch_near_dip<float, false>(S, gnode, gstart, gcount, ng, tx, ty, tz, tout, outputs, pot, grad);
+    else if (self) launch_near_dip<double, true>(S, gnode, gstart, gcount, ng, tx, ty, tz, tout, outputs, pot, grad);
+    else launch_near_dip<double, false>(S, gnode, gstart, gcount, ng, tx, ty, tz, tout, outputs, pot, grad);
     return;
   }
   if (S.plan->cache->kernel == FMMB_KERNEL_YUKAWA3D) {   // the near field in FP64 on both paths
-    if (self) launch_near<double, true, true>(S, gnode, gstart, gcount, ng, tx, ty, tz, tout, outputs, pot, grad);
-    else launch_near<double, false, true>(S, gnode, gstart, gcount, ng, tx, ty, tz, tout, outputs, pot, grad);
+    if (self) launch_near<double, true, 1>(S, gnode, gstart, gcount, ng, tx, ty, tz, tout, outputs, pot, grad);
+    else launch_near<double, false, 1>(S, gnode, gstart, gcount, ng, tx, ty, tz, tout, outputs, pot, grad);
     return;
   }
   if (mixed && self) launch_near<float, true>(S, gnode, gstart, gcount, ng, tx, ty, tz, tout, outputs, pot, grad);

@@ -180,8 +180,6 @@ struct Plan {
 struct State {
   Plan* plan = nullptr;
   int precision = FMMB_PRECISION_FP64;
-  // the launch shape chosen by the tuner (tune.cu): near-field warps per CTA (4 or 8)
-  int near_warps = 4;
   DBuf<double> xs, ys, zs, q;             // sources and charges in tree order
   DBuf<double> f3;                        // Stokeslet states: the forces in tree order (fx, fy, fz)
   DBuf<double> sd;                        //   stresslet strengths, stressvecs, doublets (3 × N planar each)
@@ -226,13 +224,12 @@ void build_tree(Plan& P, const double* xyz_dev, int ppl, int max_levels);
 // lists.cu
 void build_lists(Plan& P);
 void build_blocks(Plan& P, int TB);       // the M2L blocks of TB targets (re)cut from P.h_pair_count
-// tune.cu: the tuned launch shapes of plans and states of a kind (method, kernel, p, precision,
-// N rounded down to a power of two); 0 / unchanged where none was tuned
+// tune.cu: the tuned M2L block size of plans of a kind (method, kernel, p, N rounded down to a power of
+// two); 0 where none was tuned
 int tuned_block_size(const Plan& P);
-void apply_tuned_state(State& S);
 // times the launch shapes on the state's inputs, keeps the fastest for its kind and applies them
 // (tune_blocks: also the plan's M2L block size, shared by the plan's other states); out: the
-// chosen block size, 0, near-field warps, and the M2L and near-field ms
+// chosen block size, 0, 4 (warps of a near-field team), and the M2L and near-field ms
 void autotune(State& S, const double* xyz_dev, const double* tau_dev, bool tune_blocks, double* out);
 void build_target_pairs(Plan& P);
 // passes.cu

@@ -17,7 +17,7 @@
 // 2c(d·f)/r³ and 4c[(f·ν)/r³ − 3(d·f)(d·ν)/r⁵] (a doublet has none).
 #include <type_traits>
 
-#include "passes.cuh"
+#include "near.cuh"
 
 namespace fmmb {
 namespace {
@@ -231,11 +231,7 @@ __global__ void __launch_bounds__(GW * 32) k_stokes_l2p_grad(const int* __restri
   }
 }
 
-struct alignas(16) S8 { double x, y, z, fx, fy, fz, pad0, pad1; };
-struct alignas(16) S16 { double x, y, z, fx, fy, fz, sx, sy, sz, nx, ny, nz, gx, gy, gz, pad; };
-
-// the near field: the sources of the 27 colleagues, flattened into batches of 32 staged per warp
-// (the next batch's loads in flight), lanes over the targets; adds c·Σ to the velocities (OUT 0),
+// The near field (near.cuh): adds c·Σ to the velocities (OUT 0),
 // the pressures (OUT 1) or the velocity gradients (OUT 2, ∂u_i/∂t_j at 9·o + 3i + j). DENS adds
 // the stresslets and doublets of sd (3 × n planar: strengths, stressvecs, doublets) to the
 // Stokeslets (src/sources.jl:203-281):
@@ -243,147 +239,93 @@ struct alignas(16) S16 { double x, y, z, fx, fy, fz, sx, sy, sz, nx, ny, nz, gx,
 //   ∂u_i/∂t_j = c[d_i(A d_j + v_j) + w_i d_j + B δ_ij] with A = −3(d·f)/r⁵ + (30(d·f_s)(d·ν) + 15(d·g))/r⁷,
 //   B = (d·f)/r³ − (6(d·f_s)(d·ν) + 3(d·g))/r⁵, v = f/r³ − 6((d·ν) f_s + (d·f_s) ν)/r⁵ − 3g/r⁵,
 //   w = −f/r³ − 3g/r⁵ (the closed forms of the three gradients, summed)
-template <bool SELF, bool DENS, int OUT>
-__global__ void __launch_bounds__(SW * 32) k_stokes_near(const int* __restrict__ gnode, const int* __restrict__ gstart,
-                                                         const int* __restrict__ gcount, int ngroups,
-                                                         const double* __restrict__ tx, const double* __restrict__ ty,
-                                                         const double* __restrict__ tz, const int* __restrict__ tout,
-                                                         const double* __restrict__ xs, const double* __restrict__ ys,
-                                                         const double* __restrict__ zs, const double* __restrict__ f3,
-                                                         const double* __restrict__ sd, int64_t n,
-                                                         const int* __restrict__ plo, const int* __restrict__ phi,
-                                                         const int* __restrict__ col, double* __restrict__ out) {
-  using SV = std::conditional_t<DENS, S16, S8>;
-  __shared__ SV stg[SW][2][32];
-  __shared__ int s_lo[SW][32], s_pre[SW][32];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int grp = blockIdx.x * SW + warp;
-  if (grp >= ngroups) return;
-  const int leaf = gnode[grp];
-  const int cn = lane < NCOL ? col[(int64_t)leaf * NCOL + lane] : -1;
-  int lo = 0, len = 0;
-  if (cn >= 0) {
-    lo = plo[cn];
-    len = max(0, phi[cn] - lo + 1);
-  }
-  int incl = len;
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, o);
-    if (lane >= o) incl += v;
-  }
-  const int S = __shfl_sync(0xffffffffu, incl, 31);
-  s_lo[warp][lane] = lo;
-  s_pre[warp][lane] = incl - len;
-  const unsigned selfm = __ballot_sync(0xffffffffu, cn == leaf);
-  const int slot = selfm ? __ffs(selfm) - 1 : 0;
-  const int pself = selfm ? __shfl_sync(0xffffffffu, incl - len, slot) : -1;
-  const int loself = __shfl_sync(0xffffffffu, lo, slot), lenself = selfm ? __shfl_sync(0xffffffffu, len, slot) : 0;
-  __syncwarp();
-  auto load = [&](int b, SV& v) {
-    const int f = 32 * b + lane;
-    v = SV{};
-    if (f < S) {
-      int idx = 0;
-#pragma unroll
-      for (int step = 16; step; step >>= 1)
-        if (s_pre[warp][idx + step] <= f) idx += step;
-      const int64_t j = s_lo[warp][idx] + (f - s_pre[warp][idx]);
-      if constexpr (DENS)
-        v = SV{xs[j],         ys[j],         zs[j],         f3[j],         f3[n + j],     f3[2 * n + j],
-               sd[j],         sd[n + j],     sd[2 * n + j], sd[3 * n + j], sd[4 * n + j], sd[5 * n + j],
-               sd[6 * n + j], sd[7 * n + j], sd[8 * n + j], 0};
-      else
-        v = SV{xs[j], ys[j], zs[j], f3[j], f3[n + j], f3[2 * n + j], 0, 0};
-    }
+template <bool DENS, int OUT>
+struct StokesNear {
+  using Real = double;
+  static constexpr bool REL = false;
+  static constexpr int NA = OUT == 2 ? 9 : (OUT == 1 ? 1 : 3), CH = DENS || OUT == 2 ? 1 : 2, MINB = 4;
+  struct Args {
+    const double *xs, *ys, *zs, *f3, *sd;
+    int64_t n;
+    double* out;
   };
-  const int t0 = gstart[grp], nt = gcount[grp];
-  for (int base = 0; base < nt; base += 32) {
-    const int k = t0 + base + lane;
-    const bool act = base + lane < nt;
-    const double x = act ? tx[k] : 0.0, y = act ? ty[k] : 0.0, z = act ? tz[k] : 0.0;
-    const int fself = SELF && act && selfm ? pself + (k - loself) : -1;
-    double ux = 0, uy = 0, uz = 0;
-    double gr[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-    SV nxt;
-    load(0, nxt);
-    for (int b = 0; 32 * b < S; ++b) {
-      SV* st = stg[warp][b & 1];
-      st[lane] = nxt;
-      __syncwarp();
-      if (32 * (b + 1) < S) load(b + 1, nxt);
-      const int m = min(32, S - 32 * b);
-      const bool chk = SELF && selfm && 32 * b < pself + lenself && 32 * b + 32 > pself;   // uniform
-      const int is = fself - 32 * b;
-      for (int i = 0; i < m; ++i) {
-        const SV sv = st[i];
-        const double dx = x - sv.x, dy = y - sv.y, dz = z - sv.z;
-        const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-        double ir = rsqrt(r2);
-        if (chk && i == is) ir = 0.0;
-        const double ir3 = ir * ir * ir;
-        const double df = dx * sv.fx + dy * sv.fy + dz * sv.fz;
-        if constexpr (OUT == 2) {
-          const double ir2 = ir * ir, ir5 = ir3 * ir2;
-          const double d[3] = {dx, dy, dz};
-          double A = -3.0 * df * ir5, B = df * ir3;
-          double v[3] = {sv.fx * ir3, sv.fy * ir3, sv.fz * ir3}, w[3] = {-v[0], -v[1], -v[2]};
-          if constexpr (DENS) {
-            const double ds = dx * sv.sx + dy * sv.sy + dz * sv.sz, dn = dx * sv.nx + dy * sv.ny + dz * sv.nz;
-            const double dg = dx * sv.gx + dy * sv.gy + dz * sv.gz;
-            A += (30.0 * ds * dn + 15.0 * dg) * ir5 * ir2;
-            B -= (6.0 * ds * dn + 3.0 * dg) * ir5;
-            const double fs[3] = {sv.sx, sv.sy, sv.sz}, nu[3] = {sv.nx, sv.ny, sv.nz}, g[3] = {sv.gx, sv.gy, sv.gz};
-#pragma unroll
-            for (int e = 0; e < 3; ++e) {
-              v[e] -= (6.0 * (dn * fs[e] + ds * nu[e]) + 3.0 * g[e]) * ir5;
-              w[e] -= 3.0 * g[e] * ir5;
-            }
-          }
-#pragma unroll
-          for (int a = 0; a < 3; ++a) {
-#pragma unroll
-            for (int b = 0; b < 3; ++b) gr[a][b] += d[a] * (A * d[b] + v[b]) + w[a] * d[b] + (a == b ? B : 0.0);
-          }
-        } else if constexpr (DENS) {
-          const double ir5 = ir3 * ir * ir;
-          const double ds = dx * sv.sx + dy * sv.sy + dz * sv.sz, dn = dx * sv.nx + dy * sv.ny + dz * sv.nz;
-          if constexpr (OUT == 1) {
-            const double sn = sv.sx * sv.nx + sv.sy * sv.ny + sv.sz * sv.nz;
-            ux += 2.0 * df * ir3 + 4.0 * sn * ir3 - 12.0 * ds * dn * ir5;
-          } else {
-            const double dg = dx * sv.gx + dy * sv.gy + dz * sv.gz;
-            const double c = df * ir3 - (3.0 * dg + 6.0 * ds * dn) * ir5;
-            ux += sv.fx * ir + sv.gx * ir3 + dx * c;
-            uy += sv.fy * ir + sv.gy * ir3 + dy * c;
-            uz += sv.fz * ir + sv.gz * ir3 + dz * c;
-          }
-        } else if constexpr (OUT == 1) {
-          ux += 2.0 * df * ir3;
-        } else {
-          const double c = df * ir3;
-          ux += sv.fx * ir + dx * c;
-          uy += sv.fy * ir + dy * c;
-          uz += sv.fz * ir + dz * c;
-        }
-      }
-    }
-    if (act) {
-      const int o = tout[k];
-      if (OUT == 2) {
-#pragma unroll
-        for (int e = 0; e < 9; ++e) out[9 * (int64_t)o + e] += KSTOKES * gr[e / 3][e % 3];
-      } else if (OUT == 1) {
-        out[o] += KSTOKES * ux;
-      } else {
-        out[3 * (int64_t)o] += KSTOKES * ux;
-        out[3 * (int64_t)o + 1] += KSTOKES * uy;
-        out[3 * (int64_t)o + 2] += KSTOKES * uz;
-      }
-    }
-    __syncwarp();
+  struct alignas(16) S8 { double x, y, z, fx, fy, fz; };
+  struct alignas(16) S16 { double x, y, z, fx, fy, fz, sx, sy, sz, nx, ny, nz, gx, gy, gz, pad; };
+  using SV = std::conditional_t<DENS, S16, S8>;
+  using Src = SV;
+  struct Stage { SV s[32]; };
+  static __device__ __forceinline__ void load(const Args& a, int j, Src& v) {
+    const int64_t n = a.n;
+    if constexpr (DENS)
+      v = SV{a.xs[j],         a.ys[j],         a.zs[j],         a.f3[j],         a.f3[n + j],     a.f3[2 * n + j],
+             a.sd[j],         a.sd[n + j],     a.sd[2 * n + j], a.sd[3 * n + j], a.sd[4 * n + j], a.sd[5 * n + j],
+             a.sd[6 * n + j], a.sd[7 * n + j], a.sd[8 * n + j], 0};
+    else
+      v = SV{a.xs[j], a.ys[j], a.zs[j], a.f3[j], a.f3[n + j], a.f3[2 * n + j]};
   }
-}
+  static __device__ __forceinline__ void stage(Stage& st, int lane, const Src& v, double, double, double) { st.s[lane] = v; }
+  template <bool CHECK>
+  static __device__ __forceinline__ void batch(const Args&, const Stage& st, int m, int is, int part, int f,
+                                               const double (&t)[3], double (&acc)[NA]) {
+#pragma unroll 2
+    for (int i = part; i < m; i += f) {
+      const SV sv = st.s[i];
+      const double dx = t[0] - sv.x, dy = t[1] - sv.y, dz = t[2] - sv.z;
+      const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+      double ir = rsqrt_h(r2);
+      if (CHECK && i == is) ir = 0.0;
+      const double ir3 = ir * ir * ir;
+      const double df = dx * sv.fx + dy * sv.fy + dz * sv.fz;
+      if constexpr (OUT == 2) {
+        const double ir2 = ir * ir, ir5 = ir3 * ir2;
+        const double d[3] = {dx, dy, dz};
+        double A = -3.0 * df * ir5, B = df * ir3;
+        double v[3] = {sv.fx * ir3, sv.fy * ir3, sv.fz * ir3}, w[3] = {-v[0], -v[1], -v[2]};
+        if constexpr (DENS) {
+          const double ds = dx * sv.sx + dy * sv.sy + dz * sv.sz, dn = dx * sv.nx + dy * sv.ny + dz * sv.nz;
+          const double dg = dx * sv.gx + dy * sv.gy + dz * sv.gz;
+          A += (30.0 * ds * dn + 15.0 * dg) * ir5 * ir2;
+          B -= (6.0 * ds * dn + 3.0 * dg) * ir5;
+          const double fs[3] = {sv.sx, sv.sy, sv.sz}, nu[3] = {sv.nx, sv.ny, sv.nz}, g[3] = {sv.gx, sv.gy, sv.gz};
+#pragma unroll
+          for (int e = 0; e < 3; ++e) {
+            v[e] -= (6.0 * (dn * fs[e] + ds * nu[e]) + 3.0 * g[e]) * ir5;
+            w[e] -= 3.0 * g[e] * ir5;
+          }
+        }
+#pragma unroll
+        for (int a = 0; a < 3; ++a) {
+#pragma unroll
+          for (int b = 0; b < 3; ++b) acc[3 * a + b] += d[a] * (A * d[b] + v[b]) + w[a] * d[b] + (a == b ? B : 0.0);
+        }
+      } else if constexpr (DENS) {
+        const double ir5 = ir3 * ir * ir;
+        const double ds = dx * sv.sx + dy * sv.sy + dz * sv.sz, dn = dx * sv.nx + dy * sv.ny + dz * sv.nz;
+        if constexpr (OUT == 1) {
+          const double sn = sv.sx * sv.nx + sv.sy * sv.ny + sv.sz * sv.nz;
+          acc[0] += 2.0 * df * ir3 + 4.0 * sn * ir3 - 12.0 * ds * dn * ir5;
+        } else {
+          const double dg = dx * sv.gx + dy * sv.gy + dz * sv.gz;
+          const double c = df * ir3 - (3.0 * dg + 6.0 * ds * dn) * ir5;
+          acc[0] += sv.fx * ir + sv.gx * ir3 + dx * c;
+          acc[1] += sv.fy * ir + sv.gy * ir3 + dy * c;
+          acc[2] += sv.fz * ir + sv.gz * ir3 + dz * c;
+        }
+      } else if constexpr (OUT == 1) {
+        acc[0] += 2.0 * df * ir3;
+      } else {
+        const double c = df * ir3;
+        acc[0] += sv.fx * ir + dx * c;
+        acc[1] += sv.fy * ir + dy * c;
+        acc[2] += sv.fz * ir + dz * c;
+      }
+    }
+  }
+  static __device__ __forceinline__ void write(const Args& a, int o, const double (&acc)[NA]) {
+#pragma unroll
+    for (int e = 0; e < NA; ++e) a.out[NA * (int64_t)o + e] += KSTOKES * acc[e];
+  }
+};
 
 template <int P>
 void launch_stokes_l2p(State& S, const int* gnode, const int* gstart, const int* gcount, int ng, const double* tx,
@@ -466,16 +408,16 @@ void stokes_evaluate_groups(State& S, const int* gnode, const int* gstart, const
     default: throw Error(FMMB_ERR_UNSUPPORTED, "p out of range");
   }
   const bool d = S.stokes_dens;
-  using K = decltype(&k_stokes_near<true, true, 0>);
-  const K table[2][2][3] = {{{k_stokes_near<false, false, 0>, k_stokes_near<false, false, 1>, k_stokes_near<false, false, 2>},
-                             {k_stokes_near<false, true, 0>, k_stokes_near<false, true, 1>, k_stokes_near<false, true, 2>}},
-                            {{k_stokes_near<true, false, 0>, k_stokes_near<true, false, 1>, k_stokes_near<true, false, 2>},
-                             {k_stokes_near<true, true, 0>, k_stokes_near<true, true, 1>, k_stokes_near<true, true, 2>}}};
-  const K kern = table[self][d][output];
-  kern<<<(ng + SW - 1) / SW, SW * 32, 0, P.ctx->stream>>>(gnode, gstart, gcount, ng, tx, ty, tz, tout, S.xs.p, S.ys.p,
-                                                          S.zs.p, S.f3.p, d ? S.sd.p : nullptr, P.N, P.plo.p, P.phi.p,
-                                                          P.col.p, out);
-  FMMB_LAUNCH_CHECK();
+  const NearArgs A{gnode, gstart, gcount, ng, tx, ty, tz, tout, P.cell.p, P.plo.p, P.phi.p, P.col.p, geometry(P)};
+  auto go = [&](auto pol) {
+    using Pol = decltype(pol);
+    const typename Pol::Args pa{S.xs.p, S.ys.p, S.zs.p, S.f3.p, d ? S.sd.p : nullptr, P.N, out};
+    if (self) launch_near_leaves<Pol, true>(A, pa, P.ctx->num_sms, P.ctx->stream);
+    else launch_near_leaves<Pol, false>(A, pa, P.ctx->num_sms, P.ctx->stream);
+  };
+  if (output == FMMB_STOKES_VELOCITY) d ? go(StokesNear<true, 0>{}) : go(StokesNear<false, 0>{});
+  else if (output == FMMB_STOKES_PRESSURE) d ? go(StokesNear<true, 1>{}) : go(StokesNear<false, 1>{});
+  else d ? go(StokesNear<true, 2>{}) : go(StokesNear<false, 2>{});
 }
 
 }  // namespace

@@ -1,16 +1,15 @@
 // The autotuner of the launch shapes: tile and block shapes chosen by timing them on the
 // caller's own inputs (the reference has no tuner).
 //
-// Two shapes are free, in that no result depends on them (each target's sums are taken in the
-// list's order whatever the blocking, and a near-field warp owns its leaf group):
+// One shape is free, in that no result depends on it (each target's sums are taken in the list's
+// order whatever the blocking):
 //   - the targets per M2L block (32, 64 or 128; a plan property: its blocks are re-cut from the
-//     pairs per target), for both M2L kernels;
-//   - the near-field warps per CTA (4 or 8).
+//     pairs per target), for both M2L kernels.
 // fmmb_autotune times each candidate on the state's own inputs (CUDA events on the context's
 // stream, the median of three after one warm-up), keeps the fastest, applies it, and records it
-// for every later plan and state of the same kind: method, kernel, order, precision path and the
-// number of points rounded down to a power of two. Plans created afterwards take the recorded
-// block size; states take the recorded warps.
+// for every later plan of the same kind: method, kernel, order and the number of points rounded down
+// to a power of two. Plans created afterwards take the recorded
+// block size.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -22,9 +21,9 @@ namespace fmmb {
 namespace {
 
 struct Tuned {
-  int tb = 0, near_w = 4;
+  int tb = 0;
 };
-using Kind = std::tuple<int, int, int, int, int>;   // method, kernel, p, precision (-1: any), log2 N
+using Kind = std::tuple<int, int, int, int>;   // method, kernel, p, log2 N
 
 std::mutex g_mu;
 std::map<Kind, Tuned> g_tuned;
@@ -35,9 +34,9 @@ int log2_floor(int64_t n) {
   return b;
 }
 
-Kind kind_of(const Plan& P, int precision) {
+Kind kind_of(const Plan& P) {
   const Cache& C = *P.cache;
-  return Kind(C.method, C.kernel, C.p, precision, log2_floor(P.N));
+  return Kind(C.method, C.kernel, C.p, log2_floor(P.N));
 }
 
 // the median of three timed runs after one warm-up, in ms
@@ -67,15 +66,8 @@ double time_ms(cudaStream_t s, F&& f) {
 
 int tuned_block_size(const Plan& P) {
   std::lock_guard<std::mutex> lk(g_mu);
-  auto it = g_tuned.find(kind_of(P, -1));
+  auto it = g_tuned.find(kind_of(P));
   return it == g_tuned.end() ? 0 : it->second.tb;
-}
-
-void apply_tuned_state(State& S) {
-  std::lock_guard<std::mutex> lk(g_mu);
-  auto it = g_tuned.find(kind_of(*S.plan, S.precision));
-  if (it == g_tuned.end()) return;
-  S.near_warps = it->second.near_w;
 }
 
 void autotune(State& S, const double* xyz, const double* tau, bool tune_blocks, double* out) {
@@ -103,35 +95,27 @@ void autotune(State& S, const double* xyz, const double* tau, bool tune_blocks, 
     if (ms < best) { best = ms; best_tb = tb; }
   }
   if (P.TB != best_tb) build_blocks(P, best_tb);
-  // the near field at the sources (harmonic methods with charges: Laplace3D and Yukawa3D)
-  double best_near = 0;
-  int best_w = S.near_warps;
+  // the near field at the sources (harmonic methods with charges: Laplace3D and Yukawa3D), for the
+  // caller: it has no shape to choose
+  double near_ms = 0;
   if (C.kernel != FMMB_KERNEL_STOKESLET3D && P.n_leaves > 0) {
     DBuf<double> pot(P.N), grad(3 * P.N);
-    best_near = 1e300;
-    for (int w : {4, 8}) {
-      S.near_warps = w;
-      const double ms = time_ms(s, [&] { near_sources(S, FMMB_OUTPUT_POTENTIAL | FMMB_OUTPUT_GRADIENT, pot.p, grad.p, s); });
-      if (ms < best_near) { best_near = ms; best_w = w; }
-    }
+    near_ms = time_ms(s, [&] { near_sources(S, FMMB_OUTPUT_POTENTIAL | FMMB_OUTPUT_GRADIENT, pot.p, grad.p, s); });
     FMMB_CUDA(cudaStreamSynchronize(s));
   }
-  S.near_warps = best_w;
   S.built = false;                      // the timed stages left the expansions incomplete
   {
     std::lock_guard<std::mutex> lk(g_mu);
     Tuned t;
     t.tb = best_tb;
-    t.near_w = best_w;
-    g_tuned[kind_of(P, S.precision)] = t;
-    if (tune_blocks) g_tuned[kind_of(P, -1)] = t;
+    if (tune_blocks) g_tuned[kind_of(P)] = t;
   }
   if (out) {
     out[0] = best_tb;
     out[1] = 0;                          // the FP64 M2L has one chunk width
-    out[2] = best_w;
+    out[2] = 4;                          // warps of a near-field team
     out[3] = best;
-    out[4] = best_near;
+    out[4] = near_ms;
   }
 }
 

@@ -145,12 +145,11 @@ int fmmb_batch_plan_instances(const fmmb_plan* plan, int64_t* ninst, int64_t* of
 /* The autotuner (no counterpart in the reference): times the launch shapes of a state's matvec on
  * the given inputs (the plan's points, n of them, and its charges, or 3×n Stokeslets) — the M2L
  * block size (32, 64, 128 targets; when tune_blocks, re-cutting the plan's blocks, which its other
- * states share), the near field's warps per CTA — keeps the fastest
- * and applies it, and records it for later plans and states of the same method, kernel, order,
- * precision path and N rounded down to a power of two. No result depends on these shapes. The
- * state's expansions must be built again afterwards. out (may be NULL): 5 doubles, the block
- * size, 0 (kept for callers: the FP64 M2L has one chunk width), the warps, and the chosen M2L and
- * near-field times in ms. */
+ * states share) — keeps the fastest and applies it, and records it for later plans of the same
+ * method, kernel, order and N rounded down to a power of two. No result depends on it. The state's
+ * expansions must be built again afterwards. out (may be NULL): 5 doubles, the block size, 0 and 4
+ * (the FP64 M2L's chunk width and the near field's warps, which are no longer chosen), and the
+ * chosen M2L and the near-field times in ms. */
 int fmmb_autotune(fmmb_state* state, const double* xyz, const double* tau, int64_t n, int tune_blocks, double* out);
 int fmmb_autotune_dev(fmmb_state* state, const double* xyz_dev, const double* tau_dev, int64_t n, int tune_blocks,
                       double* out);
