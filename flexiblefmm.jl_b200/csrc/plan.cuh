@@ -243,7 +243,7 @@ void evaluate_sources(State& S, int outputs, double* pot_dev, double* grad_dev);
 void evaluate_targets(State& S, const double* tg_dev, int64_t nt, int outputs, double* pot_dev, double* grad_dev);
 // locate nt > 0 targets (device, 3 × nt) in the tree's leaves (FMMB_ERR_ARGUMENT outside the box)
 // and group them per leaf: S.t_x/t_y/t_z in leaf order, S.t_out their original indices, and the ng
-// groups (returned) as S.t_groups = [node; first; count] (ng each)
+// groups (returned) as S.t_groups = [node; first; count] (nt apart)
 int group_targets(State& S, const double* tg_dev, int64_t nt);
 // eval.cu: the evaluation at the sources split in two (harmonic methods with charges): the near
 // field on stream st writes the outputs, the far field (on the state's stream, after it) adds

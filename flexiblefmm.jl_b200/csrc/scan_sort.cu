@@ -80,14 +80,18 @@ __global__ void k_tile_scan(const int* __restrict__ in, int64_t n, const int* __
 // ---- radix sort
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
-constexpr int RS_ITEMS = 16;                      // per thread
-constexpr int RS_TILE = RS_THREADS * RS_ITEMS;    // 4096 keys per tile
 constexpr int RS_BINS = 256;
+// keys per thread: tiles of 4,096 keys, or of 1,024 where the larger ones would leave SMs idle (a tile's
+// scatter is a serial chain over its keys per thread)
+constexpr int RS_ITEMS_MAX = 16, RS_ITEMS_MIN = 4;
+constexpr int64_t RS_SMALL = 148ll * RS_THREADS * RS_ITEMS_MAX;
 
+template <int RS_ITEMS>
 __global__ void k_digit_hist(const uint64_t* __restrict__ keys, int64_t n, int shift, int ntiles, int* __restrict__ hist) {
   __shared__ int h[RS_BINS];
   for (int b = threadIdx.x; b < RS_BINS; b += blockDim.x) h[b] = 0;
   __syncthreads();
+  constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
   int64_t base = (int64_t)blockIdx.x * RS_TILE;
   for (int i = threadIdx.x; i < RS_TILE; i += RS_THREADS) {
     int64_t j = base + i;
@@ -97,7 +101,8 @@ __global__ void k_digit_hist(const uint64_t* __restrict__ keys, int64_t n, int s
   for (int b = threadIdx.x; b < RS_BINS; b += blockDim.x) hist[(int64_t)b * ntiles + blockIdx.x] = h[b];
 }
 
-// stable scatter of one tile: the keys of warp w are tile positions w·512 + it·32 + lane
+// stable scatter of one tile: the keys of warp w are tile positions w·32·RS_ITEMS + it·32 + lane
+template <int RS_ITEMS>
 __global__ void k_digit_scatter(const uint64_t* __restrict__ kin, const uint32_t* __restrict__ vin, int64_t n, int shift,
                                 int ntiles, const int* __restrict__ offs, uint64_t* __restrict__ kout,
                                 uint32_t* __restrict__ vout) {
@@ -105,6 +110,7 @@ __global__ void k_digit_scatter(const uint64_t* __restrict__ kin, const uint32_t
   int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   for (int b = threadIdx.x; b < RS_WARPS * RS_BINS; b += RS_THREADS) (&wc[0][0])[b] = 0;
   __syncthreads();
+  constexpr int RS_TILE = RS_THREADS * RS_ITEMS;
   int64_t base = (int64_t)blockIdx.x * RS_TILE + (int64_t)warp * (RS_ITEMS * 32);
   uint64_t key[RS_ITEMS];
   uint32_t val[RS_ITEMS];
@@ -169,7 +175,6 @@ void scan_exclusive(const int* in, int* out, int64_t n, cudaStream_t s) {
   scan_exclusive(sums.p, offs.p, ntiles, s);
   k_tile_scan<<<(unsigned)ntiles, SCAN_THREADS, 0, s>>>(in, n, offs.p, out);
   FMMB_LAUNCH_CHECK();
-  FMMB_CUDA(cudaStreamSynchronize(s));   // the temporaries are freed on return
 }
 
 int64_t scan_exclusive_total(const int* in, int* out, int64_t n, cudaStream_t s) {
@@ -179,22 +184,23 @@ int64_t scan_exclusive_total(const int* in, int* out, int64_t n, cudaStream_t s)
   return (int64_t)a + b;
 }
 
-void radix_sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int bits, cudaStream_t s) {
+void radix_sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int bits, cudaStream_t s, int low) {
   if (n <= 1) return;
   require(n < (1ll << 31), FMMB_ERR_ARGUMENT, "sort too large");
-  int ntiles = (int)((n + RS_TILE - 1) / RS_TILE);
+  const bool small = n < RS_SMALL;
+  const int tile = RS_THREADS * (small ? RS_ITEMS_MIN : RS_ITEMS_MAX);
+  int ntiles = (int)((n + tile - 1) / tile);
   DBuf<uint64_t> k2(n);
   DBuf<uint32_t> v2(n);
   DBuf<int> hist((size_t)RS_BINS * ntiles), offs((size_t)RS_BINS * ntiles);
   uint64_t *ka = keys, *kb = k2.p;
   uint32_t *va = vals, *vb = v2.p;
-  int passes = (bits + 7) / 8;
-  for (int ps = 0; ps < passes; ++ps) {
-    int shift = 8 * ps;
-    k_digit_hist<<<ntiles, RS_THREADS, 0, s>>>(ka, n, shift, ntiles, hist.p);
+  for (int shift = low; shift < bits; shift += 8) {
+    (small ? k_digit_hist<RS_ITEMS_MIN> : k_digit_hist<RS_ITEMS_MAX>)<<<ntiles, RS_THREADS, 0, s>>>(ka, n, shift, ntiles, hist.p);
     FMMB_LAUNCH_CHECK();
     scan_exclusive(hist.p, offs.p, (int64_t)RS_BINS * ntiles, s);
-    k_digit_scatter<<<ntiles, RS_THREADS, 0, s>>>(ka, va, n, shift, ntiles, offs.p, kb, vb);
+    (small ? k_digit_scatter<RS_ITEMS_MIN> : k_digit_scatter<RS_ITEMS_MAX>)<<<ntiles, RS_THREADS, 0, s>>>(
+        ka, va, n, shift, ntiles, offs.p, kb, vb);
     FMMB_LAUNCH_CHECK();
     std::swap(ka, kb);
     std::swap(va, vb);
@@ -203,7 +209,6 @@ void radix_sort_pairs(uint64_t* keys, uint32_t* vals, int64_t n, int bits, cudaS
     FMMB_CUDA(cudaMemcpyAsync(keys, ka, n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
     FMMB_CUDA(cudaMemcpyAsync(vals, va, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s));
   }
-  FMMB_CUDA(cudaStreamSynchronize(s));
 }
 
 }  // namespace fmmb

@@ -436,7 +436,7 @@ void stokes_evaluate_targets(State& S, const double* tg_dev, int64_t nt, int out
   if (nt == 0) return;
   const int ng = group_targets(S, tg_dev, nt);
   const int* g = S.t_groups.p;
-  stokes_evaluate_groups(S, g, g + ng, g + 2 * ng, ng, S.t_x.p, S.t_y.p, S.t_z.p, S.t_out.p, false, output, out_dev);
+  stokes_evaluate_groups(S, g, g + nt, g + 2 * nt, ng, S.t_x.p, S.t_y.p, S.t_z.p, S.t_out.p, false, output, out_dev);
 }
 
 }  // namespace fmmb
