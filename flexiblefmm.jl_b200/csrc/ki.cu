@@ -31,8 +31,7 @@ inline unsigned nblk(int64_t n, int t = 256) { return (unsigned)((n + t - 1) / t
 inline int round_up(int x, int m) { return (x + m - 1) / m * m; }
 
 constexpr int FB = 64;             // frequencies per block of the Hadamard stage
-constexpr int HAD_THREADS = 512;   // 16 warps, one target at a time each
-constexpr int HAD_UNROLL = 16;
+constexpr int HAD_THREADS = 512;   // 16 warps, one sibling group at a time each
 constexpr int SIDE = 2 * KI_PMAX;
 
 
@@ -106,13 +105,16 @@ __global__ void __launch_bounds__(128) k_ki_check(const int* __restrict__ nodes,
 
 // ---------------------------------------------------------------- the spectral M2L
 // forward: the density of node g (its ns small-surface values, embedded in the p³ corner of the
-// (2p)³ lattice) to its half spectrum, separable DFTs in shared memory
+// (2p)³ lattice) to its half spectrum, separable DFTs in shared memory; nodes without sources are no
+// pair's source and need none (about half the nodes of the adaptive configuration)
 __global__ void __launch_bounds__(128) k_ki_forward(int first, int p, int ns, int LD, int nfp,
-                                                    const double* __restrict__ M, const float2* __restrict__ tw,
-                                                    const int* __restrict__ embed, float2* __restrict__ spec) {
+                                                    const uint8_t* __restrict__ flags, const double* __restrict__ M,
+                                                    const float2* __restrict__ tw, const int* __restrict__ embed,
+                                                    float2* __restrict__ spec) {
   extern __shared__ float2 smf[];
   __shared__ float2 c_tw[SIDE * SIDE];              // [j·n + k] = e^{−2πi jk/n}, n = 2p
   const int g = first + blockIdx.x, n = 2 * p, nh = p + 1, tid = threadIdx.x;
+  if (!(flags[g] & F_SOURCE)) return;
   float2* a1 = smf;                                 // [nh·p·p]
   float2* a2 = a1 + nh * p * p;                     // [nh·n·p]
   float* x = reinterpret_cast<float*>(a2 + nh * n * p);   // [p³]
@@ -166,53 +168,97 @@ __global__ void __launch_bounds__(128) k_ki_forward(int first, int p, int ns, in
   }
 }
 
-// Hadamard sums: CTA (frequency block fb, range of targets); the 316 tables' block fb in shared
-// memory; a warp per target, lane l the frequencies 2l, 2l + 1 of the block
-__global__ void __launch_bounds__(HAD_THREADS) k_ki_hadamard(int first, int last, int per_cta, int nfp,
-                                                             const int* __restrict__ ptr, const int2* __restrict__ tp,
+// two FP32 multiply-adds per instruction (f32x2)
+__device__ __forceinline__ uint64_t ki_pk(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 ki_upk(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ void ki_fma2(uint64_t& d, uint64_t a, uint64_t b) {
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
+// Hadamard sums: CTA (frequency block fb, range of sibling groups); the 316 tables' block fb in shared
+// memory; a warp per group, lane l the frequencies 2l, 2l + 1 of the block. The eight siblings' far
+// sources are the sourced children of their parent's colleagues, so each source's spectrum is read once
+// and multiplied into every sibling it is far from (seven of eight on average, in registers): what
+// bounds the sums is the L1 / shared-memory pipe, and a pair moves one table entry and an eighth of a
+// spectrum through it in place of one of each, with half the multiply-add instructions (f32x2).
+// fidx: per colleague offset (27), source child and target child the far offset's index, −1 when near.
+__global__ void __launch_bounds__(HAD_THREADS) k_ki_hadamard(int ngroups, int per_cta, int nfp,
+                                                             const int2* __restrict__ groups,
+                                                             const int* __restrict__ ptr, const int4* __restrict__ cell,
+                                                             const int* __restrict__ cf, const int* __restrict__ col,
+                                                             const uint8_t* __restrict__ flags,
+                                                             const int16_t* __restrict__ fidx,
                                                              const float2* __restrict__ tab,
                                                              const float2* __restrict__ spec, float2* __restrict__ U) {
-  extern __shared__ float4 st[];   // [NFAR][FB / 2]
+  extern __shared__ float4 st[];   // [NFAR][FB / 2]: (re, re, im, im) of a frequency pair
+  int16_t* sf = reinterpret_cast<int16_t*>(st + NFAR * (FB / 2));   // [27][8][8]
   const int fb = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   for (int i = tid; i < NFAR * (FB / 2); i += HAD_THREADS) {
     const int f = i / (FB / 2), l = i % (FB / 2);
-    st[i] = reinterpret_cast<const float4*>(tab + (int64_t)f * nfp + fb * FB)[l];
+    const float4 v = reinterpret_cast<const float4*>(tab + (int64_t)f * nfp + fb * FB)[l];
+    st[i] = make_float4(v.x, v.z, v.y, v.w);
   }
+  for (int i = tid; i < NCOL * NCH * NCH; i += HAD_THREADS) sf[i] = fidx[i];
   __syncthreads();
-  const int t0 = first + blockIdx.y * per_cta, t1 = min(last, t0 + per_cta);
-  for (int t = t0 + warp; t < t1; t += HAD_THREADS / 32) {
-    const int k0 = ptr[t], k1 = ptr[t + 1];
-    if (k0 == k1) continue;
-    float ar = 0.f, ai = 0.f, br = 0.f, bi = 0.f;
-    int k = k0;
-    // HAD_UNROLL pairs' loads in flight per warp: the kernel is bound by their latency
-    for (; k + HAD_UNROLL <= k1; k += HAD_UNROLL) {
-      int2 pr[HAD_UNROLL];
-      float4 sv[HAD_UNROLL];
+  const int q0 = blockIdx.y * per_cta, q1 = min(ngroups, q0 + per_cta);
+  for (int q = q0 + warp; q < q1; q += HAD_THREADS / 32) {
+    const int2 gr = groups[q];                       // parent, first sibling
+    if (ptr[gr.y] == ptr[gr.y + NCH]) continue;      // no far pairs
+    // lane k: colleague k of the parent, its children and which of them have sources
+    int s0 = -1, o = 0, mask = 0;
+    if (lane < NCOL) {
+      const int pc = col[(int64_t)gr.x * NCOL + lane];
+      if (pc >= 0) {
+        s0 = cf[pc];
+        const int4 a = cell[pc], b = cell[gr.x];
+        o = (a.x - b.x + 1) + 3 * (a.y - b.y + 1) + 9 * (a.z - b.z + 1);
+      }
+      if (s0 >= 0)
+        for (int b = 0; b < NCH; ++b) mask |= ((flags[s0 + b] & F_SOURCE) != 0) << b;
+    }
+    uint64_t ur[NCH], ui[NCH];
 #pragma unroll
-      for (int u = 0; u < HAD_UNROLL; ++u) pr[u] = tp[k + u];
+    for (int a = 0; a < NCH; ++a) ur[a] = ui[a] = 0;
+    for (unsigned left = __ballot_sync(0xffffffffu, mask != 0); left; left &= left - 1) {
+      const int k = __ffs(left) - 1;
+      const int s = __shfl_sync(0xffffffffu, s0, k), ok = __shfl_sync(0xffffffffu, o, k), mk = __shfl_sync(0xffffffffu, mask, k);
+      const float2* src = spec + (int64_t)s * nfp + fb * FB + 2 * lane;
+      float4 v[NCH];
 #pragma unroll
-      for (int u = 0; u < HAD_UNROLL; ++u)
-        sv[u] = __ldg(reinterpret_cast<const float4*>(spec + (int64_t)pr[u].x * nfp + fb * FB) + lane);
+      for (int b = 0; b < NCH; ++b)
+        if ((mk >> b) & 1) v[b] = __ldg(reinterpret_cast<const float4*>(src + (int64_t)b * nfp));
+      const uint4* fi = reinterpret_cast<const uint4*>(sf + ok * NCH * NCH);
 #pragma unroll
-      for (int u = 0; u < HAD_UNROLL; ++u) {
-        const float4 tv = st[pr[u].y * (FB / 2) + lane];
-        ar = fmaf(tv.x, sv[u].x, fmaf(-tv.y, sv[u].y, ar));
-        ai = fmaf(tv.x, sv[u].y, fmaf(tv.y, sv[u].x, ai));
-        br = fmaf(tv.z, sv[u].z, fmaf(-tv.w, sv[u].w, br));
-        bi = fmaf(tv.z, sv[u].w, fmaf(tv.w, sv[u].z, bi));
+      for (int b = 0; b < NCH; ++b) {
+        if (!((mk >> b) & 1)) continue;              // uniform
+        const uint64_t xr = ki_pk(v[b].x, v[b].z), xi = ki_pk(v[b].y, v[b].w), nx = ki_pk(-v[b].y, -v[b].w);
+        const uint4 fw = fi[b];
+        const uint32_t w[4] = {fw.x, fw.y, fw.z, fw.w};
+#pragma unroll
+        for (int a = 0; a < NCH; ++a) {
+          const int f = (int)(int16_t)(w[a >> 1] >> (16 * (a & 1)));
+          if (f < 0) continue;                       // uniform
+          const ulonglong2 t = reinterpret_cast<const ulonglong2*>(st)[f * (FB / 2) + lane];
+          ki_fma2(ur[a], t.x, xr);
+          ki_fma2(ur[a], t.y, nx);
+          ki_fma2(ui[a], t.x, xi);
+          ki_fma2(ui[a], t.y, xr);
+        }
       }
     }
-    for (; k < k1; ++k) {
-      const int2 pr = tp[k];
-      const float4 sv = __ldg(reinterpret_cast<const float4*>(spec + (int64_t)pr.x * nfp + fb * FB) + lane);
-      const float4 tv = st[pr.y * (FB / 2) + lane];
-      ar = fmaf(tv.x, sv.x, fmaf(-tv.y, sv.y, ar));
-      ai = fmaf(tv.x, sv.y, fmaf(tv.y, sv.x, ai));
-      br = fmaf(tv.z, sv.z, fmaf(-tv.w, sv.w, br));
-      bi = fmaf(tv.z, sv.w, fmaf(tv.w, sv.z, bi));
+#pragma unroll
+    for (int a = 0; a < NCH; ++a) {
+      const float2 r = ki_upk(ur[a]), i = ki_upk(ui[a]);
+      reinterpret_cast<float4*>(U + (int64_t)(gr.y + a) * nfp + fb * FB)[lane] = make_float4(r.x, i.x, r.y, i.y);
     }
-    reinterpret_cast<float4*>(U + (int64_t)t * nfp + fb * FB)[lane] = make_float4(ar, ai, br, bi);
   }
 }
 
@@ -323,6 +369,21 @@ void ki_prepare(Plan& P) {
         tw[k] = make_float2((float)std::cos(2 * M_PI * k / n), (float)-std::sin(2 * M_PI * k / n));
       to_device(C.ki_tw, tw, s);
       to_device(C.ki_embed, h->embed, s);
+      // the far offset of child b of the colleague at offset o from child a of the box, −1 when near
+      std::vector<int> far(343, -1);
+      for (int f = 0; f < NFAR; ++f) {
+        const int8_t* x = &C.host.faroff[3 * f];
+        far[(x[0] + 3) + 7 * (x[1] + 3) + 49 * (x[2] + 3)] = f;
+      }
+      std::vector<int16_t> fidx(NCOL * NCH * NCH);
+      for (int o = 0; o < NCOL; ++o)
+        for (int b = 0; b < NCH; ++b)
+          for (int a = 0; a < NCH; ++a) {
+            const int x = 2 * (o % 3 - 1) + (b & 1) - (a & 1), y = 2 * (o / 3 % 3 - 1) + (b >> 1 & 1) - (a >> 1 & 1),
+                      z = 2 * (o / 9 - 1) + (b >> 2) - (a >> 2);
+            fidx[(o * NCH + b) * NCH + a] = (int16_t)far[(x + 3) + 7 * (y + 3) + 49 * (z + 3)];
+          }
+      to_device(C.ki_fidx, fidx, s);
       FMMB_CUDA(cudaStreamSynchronize(s));
       C.ki = h;
     }
@@ -330,6 +391,14 @@ void ki_prepare(Plan& P) {
   P.lv_m2m.assign(P.L, C.ki_m2m.p);
   P.lv_l2l.assign(P.L, C.ki_l2l.p);
   build_target_pairs(P);
+  std::vector<int2> groups;                 // the sibling groups of the levels with far pairs
+  for (int l = 2; l < P.L; ++l)
+    for (int g = 0; g < P.level_groups[l]; ++g) {
+      const int c0 = P.level_start[l] + NCH * g;
+      groups.push_back(make_int2(P.h_parent[c0], c0));
+    }
+  P.n_ki_groups = (int)groups.size();
+  to_device(P.ki_groups, groups, s);
   // every real leaf, sources or not: evaluate() may locate targets in the empty ones
   std::vector<int> all;
   for (int g = 0; g < P.nnodes; ++g)
@@ -378,14 +447,18 @@ int ki_m2l(State& S) {
   const int p = C.p, n = 2 * p, nh = p + 1;
   const size_t fsm = sizeof(float2) * (nh * p * p + nh * n * p) + sizeof(float) * p * p * p;
   FMMB_CUDA(cudaFuncSetAttribute(k_ki_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm));
-  k_ki_forward<<<nt, 128, fsm, s>>>(first, p, C.np, C.ld, C.ki_nfp, S.M.p, C.ki_tw.p, C.ki_embed.p, S.ki_spec.p);
+  k_ki_forward<<<nt, 128, fsm, s>>>(first, p, C.np, C.ld, C.ki_nfp, P.flags.p, S.M.p, C.ki_tw.p, C.ki_embed.p,
+                                     S.ki_spec.p);
   FMMB_LAUNCH_CHECK();
-  const size_t hsm = sizeof(float4) * NFAR * (FB / 2);
+  const size_t hsm = sizeof(float4) * NFAR * (FB / 2) + sizeof(int16_t) * NCOL * NCH * NCH;
   FMMB_CUDA(cudaFuncSetAttribute(k_ki_hadamard, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm));
-  const int per_cta = 256;
-  k_ki_hadamard<<<dim3(C.ki_nfp / FB, (nt + per_cta - 1) / per_cta), HAD_THREADS, hsm, s>>>(
-      first, last, per_cta, C.ki_nfp, P.tp_ptr.p, P.tp.p, C.ki_tab.p, S.ki_spec.p, S.ki_u.p);
-  FMMB_LAUNCH_CHECK();
+  if (P.n_ki_groups > 0) {
+    const int per_cta = 64;
+    k_ki_hadamard<<<dim3(C.ki_nfp / FB, (P.n_ki_groups + per_cta - 1) / per_cta), HAD_THREADS, hsm, s>>>(
+        P.n_ki_groups, per_cta, C.ki_nfp, P.ki_groups.p, P.tp_ptr.p, P.cell.p, P.cf.p, P.col.p, P.flags.p, C.ki_fidx.p,
+        C.ki_tab.p, S.ki_spec.p, S.ki_u.p);
+    FMMB_LAUNCH_CHECK();
+  }
   const size_t ism = sizeof(float2) * (nh * n * n + nh * n * p + nh * p * p) + sizeof(float) * p * p * p;
   FMMB_CUDA(cudaFuncSetAttribute(k_ki_inverse, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ism));
   k_ki_inverse<<<nt, 128, ism, s>>>(first, p, C.np, C.ld, C.ki_nfp, P.tp_ptr.p, P.cell.p, P.W0, C.ki_tw.p, C.ki_embed.p,

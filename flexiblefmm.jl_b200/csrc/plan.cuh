@@ -80,6 +80,7 @@ struct Cache {
   DBuf<double> ki_large, ki_upv, ki_upsu, ki_downv, ki_downsu, ki_m2m, ki_l2l;
   DBuf<int> ki_embed;
   DBuf<float2> ki_tab, ki_tw;
+  DBuf<int16_t> ki_fidx;                  // far offset index by colleague offset, source child, target child
   // KernelIndependent(Laplace2D()): circle operators per width (keyed by the exponent e of
   // w = ldexp(W0, e)), built on the host when a plan first needs that width
   struct CircleLevel { DBuf<double> upv, upsu, downv, downsu, m2m, l2l, m2l; };
@@ -152,6 +153,8 @@ struct Plan {
   DBuf<int2> tp;
   DBuf<int> ki_leaves;                    // every real leaf (with sources or not)
   int n_ki_leaves = 0;
+  DBuf<int2> ki_groups;                   // the sibling groups of the levels ≥ 2: parent, first child
+  int n_ki_groups = 0;
   // the circle method: per level its pseudo-inverse factors, and the level ranges of the
   // childless nodes with sources and of the real leaves (both lists are in node order)
   std::vector<const double*> kic_upv, kic_upsu, kic_downv, kic_downsu;
