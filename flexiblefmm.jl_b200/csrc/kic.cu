@@ -64,7 +64,10 @@ __global__ void __launch_bounds__(128) k_kic_check(const int* __restrict__ nodes
 }
 
 // the dense M2L: warp per target t, Pl[t] = Σ over its far pairs (s, f) of A_f(level) · M[s]
-// (rows lane and lane + 32; the columns of M[s] broadcast by shuffles)
+// (rows lane and lane + 32; the columns of M[s] broadcast by shuffles). Only the in-plane offsets have a
+// map: the far offsets are listed by layers of oz, and those of oz = 0 are the 40 after 98 + 40 others. The
+// pairs of the embedding's off-plane boxes, half of all pairs or more, are passed over.
+constexpr int INPLANE0 = 138, INPLANE = 40;
 __global__ void __launch_bounds__(128) k_kic_m2l(int first, int last, int N, const int* __restrict__ ptr,
                                                  const int2* __restrict__ tp, const int4* __restrict__ cell,
                                                  const uint64_t* __restrict__ ops_lv, const double* __restrict__ M,
@@ -77,6 +80,7 @@ __global__ void __launch_bounds__(128) k_kic_m2l(int first, int last, int N, con
   double a0 = 0, a1 = 0;
   for (int k = k0; k < k1; ++k) {
     const int2 pr = tp[k];
+    if ((unsigned)(pr.y - INPLANE0) >= (unsigned)INPLANE) continue;
     const double* A = ops + (int64_t)pr.y * CLD * CLD;
     const double* x = M + (int64_t)pr.x * CLD;
     const double xl = x[lane], xh = x[lane + 32];
