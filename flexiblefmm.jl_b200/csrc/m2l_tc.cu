@@ -23,7 +23,14 @@
 //   - gather warps build K-step slabs of A (128 rows × 16 FP16, head and tail, in the UMMA
 //     K-major canonical layout) into a ring: 8 lanes write the 8 rows of one 128-byte core
 //     matrix; odd quarter-turn rotations read a second copy of the multipoles in which the two
-//     entries of every odd-order pair are swapped, and the source-side signs cost one XOR;
+//     entries of every odd-order pair are swapped, and the source-side signs cost one XOR on the way
+//     from the load's registers to shared memory. The gather's latency bounds the kernel (per round of
+//     128 pairs about 7,500 cycles at p = 11, of which the MMAs take 2,000), so its first loads are
+//     issued before the slab's buffer is free, and where the ring holds fewer slabs than there are
+//     gather warps two warps share a slab. Measured (one warp a slab, cp.async into the slab and the
+//     signs in place → two warps → loads through registers): a million points p = 11 1.79 → 1.71 →
+//     1.59 ms, 300,000 points of a Gaussian mixture p = 8 1.18 → 1.12 → 1.06, a sphere of 100,000 p = 6
+//     0.49 → 0.44;
 //   - one thread loads the class operator (head and tail, laid out on the host) with one bulk
 //     copy (cp.async.bulk, no tensor map, no multicast) when the class changes, after the
 //     previous class's MMAs completed; then per K-step issues three MMAs (M = 128, N, K = 16)
@@ -141,15 +148,6 @@ __device__ __forceinline__ void bulk_load(void* dst, const void* src, uint32_t b
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(smem_u32(dst)),
                "l"(src), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
-}
-
-// 16 bytes from global memory into shared memory, asynchronously (L2 only); the bytes past
-// src_bytes (0 or 16) are zero-filled
-__device__ __forceinline__ void cp_async16(void* dst, const void* src, uint32_t src_bytes) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(dst)), "l"(src), "r"(src_bytes) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() {
-  asm volatile("cp.async.commit_group;\n\tcp.async.wait_group 0;" ::: "memory");
 }
 
 // a reduction without a returned value (an atomicAdd whose result is unused may still wait for one)
@@ -277,6 +275,8 @@ struct Cfg {
   // already have seen fill k − 2·NSLAB consumed, or the wait on that barrier's phase parity could
   // pass a phase early; its previous slab k − NGW waited for k − NGW − NSLAB, so NGW ≤ NSLAB
   static constexpr int NGW = GW < NSLAB ? GW : NSLAB;
+  // the warps left over share the slabs: GPS warps build one, 128 / GPS rows each
+  static constexpr int GPS = GW / NGW >= 4 ? 4 : (GW / NGW >= 2 ? 2 : 1);
   // round records in the ring. A gather warp may work up to (RING_KSTEPS + KS − 2) / KS rounds ahead
   // of the oldest unconsumed slab's round; the ring must be longer than that, or a wait on a
   // record's phase parity could see the record's previous-but-one phase as complete
@@ -431,7 +431,7 @@ k_m2l_tc(const int4* __restrict__ blocks, const int* __restrict__ cls_off, const
     }
   }
   if (tid == 0) {
-    for (int s = 0; s < G::NSLAB; ++s) { mbar_init(&sfull[s], 1); mbar_init(&sempty[s], 1); }
+    for (int s = 0; s < G::NSLAB; ++s) { mbar_init(&sfull[s], G::GPS); mbar_init(&sempty[s], 1); }
     for (int s = 0; s < G::NREC; ++s) { mbar_init(&rfull[s], 1); mbar_init(&rempty[s], RBW); }
     for (int s = 0; s < 2; ++s) { mbar_init(&dfull[s], 1); mbar_init(&dempty[s], RBW); }
     mbar_init(opfull, 1);
@@ -489,40 +489,47 @@ k_m2l_tc(const int4* __restrict__ blocks, const int* __restrict__ cls_off, const
     int total = 0;
     for (int c = 0; c < NCLASS; ++c) total += nr[c];
     const long long nslabs = (long long)total * G::SPR;
-    for (long long k = gw; gw < G::NGW && k < nslabs && ok; k += G::NGW) {
+    constexpr int RU = 16 / G::GPS;                            // 8-row groups of this warp
+    const int u0 = gw / G::NGW * RU;
+    for (long long k = gw % G::NGW; gw < G::NGW * G::GPS && k < nslabs && ok; k += G::NGW) {
       const int i = (int)(k / G::SPR), ks0 = (int)(k % G::SPR) * G::SK, rc = i % G::NREC, s = (int)(k % G::NSLAB);
       bool w = mbar_wait_abortable(&rfull[rc], (uint32_t)(i / G::NREC) & 1, abort_flag, wns);
-      if (w && k >= G::NSLAB) w = mbar_wait_abortable(&sempty[s], (uint32_t)(k / G::NSLAB - 1) & 1, abort_flag, wns);
       if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
       const RoundRec& rec = recs[rc];
-      unsigned char* dst0 = sSlab + s * G::SLAB + half * G::SLAB_HALF + kc * CORE + o * 16;
-      // the 16 rows' chunks of the slab's K-steps copied asynchronously (zero rows where a target
-      // has no pair), then the source-side signs applied in place; odd quarter-turns read the copy
-      // with the odd-order pairs swapped
-      uint64_t facs = 0;
-      uint32_t valid = 0;
+      unsigned char* dst0 = sSlab + s * G::SLAB + half * G::SLAB_HALF + kc * CORE + o * 16 + u0 * G::SBO_A;
+      // the rows' 16-byte chunks of the slab's K-steps, UB rows' loads in flight at once (zero rows where
+      // a target has no pair; the first batch's while the slab's buffer is still in use), the source-side
+      // signs applied on the way to shared memory; odd quarter-turns read the copy with the odd-order
+      // pairs swapped
+      constexpr int UB = G::SK == 3 ? 2 : 4;                   // what 72 registers hold
+      static_assert(RU % UB == 0, "whole batches of rows");
+#pragma unroll 1
+      for (int ub = 0; ub < RU; ub += UB) {
+        uint4 v[UB][G::SK];
+        int fac[UB];
 #pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        const int row = 8 * u + o, src = rec.src[row], fac = rec.fac[row];
-        facs |= (uint64_t)fac << (4 * u);
-        valid |= (src >= 0 ? 1u : 0u) << u;
-        const uint16_t* g = src >= 0 ? Mx + (int64_t)(fac & 1) * vstride + (int64_t)src * KP + 8 * (2 * ks0 + kc) : Mx;
+        for (int u = 0; u < UB; ++u) {
+          const int row = 8 * (u0 + ub + u) + o, src = rec.src[row];
+          fac[u] = rec.fac[row];
+          const uint4* g = reinterpret_cast<const uint4*>(Mx + (int64_t)(fac[u] & 1) * vstride + (int64_t)max(src, 0) * KP +
+                                                          8 * (2 * ks0 + kc));
 #pragma unroll
-        for (int j = 0; j < G::SK; ++j) cp_async16(dst0 + u * G::SBO_A + j * 2 * CORE, g + (src >= 0 ? 16 * j : 0), src >= 0 ? 16u : 0u);
-      }
-      cp_async_wait_all();
-#pragma unroll
-      for (int u = 0; u < 16; ++u) {
-        if (!((valid >> u) & 1u)) continue;
-        const int fac = (int)((facs >> (4 * u)) & 15);
-#pragma unroll
-        for (int j = 0; j < G::SK; ++j) {
-          uint4* pv = (uint4*)(dst0 + u * G::SBO_A + j * 2 * CORE);
-          const uint4 sg = s_sgn[(2 * (ks0 + j) + kc) * 16 + fac];
-          const uint4 v = *pv;
-          *pv = make_uint4(v.x ^ sg.x, v.y ^ sg.y, v.z ^ sg.z, v.w ^ sg.w);
+          for (int j = 0; j < G::SK; ++j) v[u][j] = src >= 0 ? __ldg(g + 2 * j) : make_uint4(0u, 0u, 0u, 0u);
         }
+        if (ub == 0 && k >= G::NSLAB) {
+          w = mbar_wait_abortable(&sempty[s], (uint32_t)(k / G::NSLAB - 1) & 1, abort_flag, wns);
+          if (!__all_sync(0xffffffffu, w)) { ok = false; break; }
+        }
+#pragma unroll
+        for (int u = 0; u < UB; ++u)
+#pragma unroll
+          for (int j = 0; j < G::SK; ++j) {
+            const uint4 sg = s_sgn[(2 * (ks0 + j) + kc) * 16 + fac[u]];
+            const uint4 x = v[u][j];
+            *(uint4*)(dst0 + (ub + u) * G::SBO_A + j * 2 * CORE) = make_uint4(x.x ^ sg.x, x.y ^ sg.y, x.z ^ sg.z, x.w ^ sg.w);
+          }
       }
+      if (!ok) break;
       fence_async_smem();
       __syncwarp();
       if (lane == 0 && k != ctl.stall_slab) mbar_arrive(&sfull[s]);
