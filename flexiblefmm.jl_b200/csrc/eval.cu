@@ -21,46 +21,12 @@
 namespace fmmb {
 namespace {
 
-// The leaf's local expansion prepared for L2P (harmonics.jl:447-486): per (m, n), m-major, eight
-// values — the potential's coefficient pair and the three gradient components' pairs (each from
-// the degree-(n+1) coefficients and the recurrence tables), the factor 2 of the m ≥ 1 terms
-// folded in — so that every term of the point loop is a complex dot product a·v with the
-// regular harmonic v = Υ̃_n^m(x̂). Built once per leaf (FP64, then rounded to R).
-template <int P>
-__host__ __device__ constexpr int l2p_entries() { return (P + 1) * (P + 2) / 2; }
-__device__ __forceinline__ int l2p_entry(int P, int m, int n) { return m * (P + 1) - m * (m - 1) / 2 + n - m; }
-
+// The leaf's local expansion prepared for L2P: the entries' eight values (l2p_values), rounded to R, m-major
 template <int P, typename R>
-__device__ void l2p_prepare(const double* __restrict__ L, R* __restrict__ E, int lane) {
-  for (int q = lane; q < l2p_entries<P>(); q += 32) {
-    int m = 0, rem = q;
-    while (rem >= P + 1 - m) { rem -= P + 1 - m; ++m; }
-    const int n = m + rem;
-    double v[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    // potential: Σ L_n^m conj Υ̃ (harmonics.jl:455-462)
-    if (m == 0) v[0] = L[n * n];
-    else { v[0] = 2 * L[n * n + 2 * m - 1]; v[1] = 2 * L[n * n + 2 * m]; }
-    // gradient from degree n + 1 (harmonics.jl:465-486)
-    if (n < P) {
-      const int n1 = n + 1;
-      if (m == 0) {
-        const double cmv = ctab<double>(3 * TRI_MAX + tri(n1, 1));
-        v[2] = -cmv * L[n1 * n1 + 1];
-        v[4] = -cmv * L[n1 * n1 + 2];
-        v[6] = ctab<double>(2 * TRI_MAX + tri(n1, 0)) * L[n1 * n1];
-      } else {
-        const double ur = L[n1 * n1 + 2 * (m + 1) - 1], ui = L[n1 * n1 + 2 * (m + 1)];
-        double dr, di;
-        if (m == 1) { dr = L[n1 * n1]; di = 0; }
-        else { dr = L[n1 * n1 + 2 * (m - 1) - 1]; di = L[n1 * n1 + 2 * (m - 1)]; }
-        const double cu = 0.5 * ctab<double>(3 * TRI_MAX + tri(n1, m + 1));
-        const double cd = 0.5 * ctab<double>(4 * TRI_MAX + tri(n1, m - 1));
-        const double czv = ctab<double>(2 * TRI_MAX + tri(n1, m));
-        v[2] = 2 * (-cu * ur + cd * dr); v[3] = 2 * (-cu * ui + cd * di);
-        v[4] = -2 * (cu * ui + cd * di); v[5] = 2 * (cu * ur + cd * dr);
-        v[6] = 2 * czv * L[n1 * n1 + 2 * m - 1]; v[7] = 2 * czv * L[n1 * n1 + 2 * m];
-      }
-    }
+__device__ void l2p_prepare(const double* __restrict__ L, R* __restrict__ E, int first, int step) {
+  for (int q = first; q < l2p_entries<P>(); q += step) {
+    double v[8];
+    l2p_values<P>(L, q, v);
 #pragma unroll
     for (int i = 0; i < 8; ++i) E[8 * q + i] = (R)v[i];
   }
@@ -114,25 +80,27 @@ __global__ void __launch_bounds__(256) k_l2p(const int* __restrict__ gnode, cons
                                              const int* __restrict__ tout, const int4* __restrict__ cell,
                                              const double* __restrict__ Pl, int LD, Geometry geo,
                                              const double* __restrict__ scale, int outputs, double* __restrict__ pot,
-                                             double* __restrict__ grad, const double* __restrict__ kh2, int acc) {
+                                             double* __restrict__ grad, const double* __restrict__ kh2, int acc, int team) {
   extern __shared__ __align__(16) unsigned char sl_raw[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int grp = blockIdx.x * (blockDim.x >> 5) + warp;
+  // a leaf's entries are prepared, and its targets shared out, by `team` warps: one, or all of the CTA's
+  const int grp = team ? blockIdx.x : blockIdx.x * (blockDim.x >> 5) + warp;
   if (grp >= ngroups) return;
-  const int leaf = gnode[grp];
-  R* L = reinterpret_cast<R*>(sl_raw) + warp * (YK ? LD : 8 * l2p_entries<P>());
+  const int leaf = gnode[grp], first = team ? threadIdx.x : lane, step = team ? blockDim.x : 32;
+  R* L = reinterpret_cast<R*>(sl_raw) + (team ? 0 : warp) * (YK ? LD : 8 * l2p_entries<P>());
   if constexpr (YK) {
-    for (int i = lane; i < LD; i += 32) L[i] = (R)Pl[(int64_t)leaf * LD + i];
+    for (int i = first; i < LD; i += step) L[i] = (R)Pl[(int64_t)leaf * LD + i];
   } else {
-    l2p_prepare<P, R>(Pl + (int64_t)leaf * LD, L, lane);
+    l2p_prepare<P, R>(Pl + (int64_t)leaf * LD, L, first, step);
   }
-  __syncwarp();
+  if (team) __syncthreads();
+  else __syncwarp();
   const int4 c = cell[leaf];
   const Geometry gn = geo.at(leaf);
   const double w = ldexp(geo.W0, -c.w), s = scale[c.w];
   const double cx = gn.center(0, c.x, w), cy = gn.center(1, c.y, w), cz = gn.center(2, c.z, w);
   const int t0 = gstart[grp], nt = gcount[grp];
-  for (int base = 0; base < nt; base += 32) {
+  for (int base = first - lane; base < nt; base += step) {
     const int k = t0 + base + lane;
     const bool act = base + lane < nt;
     const double x = act ? tx[k] : cx, y = act ? ty[k] : cy, z = act ? tz[k] : cz;
@@ -548,13 +516,18 @@ void launch_l2p(State& S, const int* gnode, const int* gstart, const int* gcount
   const bool mixed = S.precision == FMMB_PRECISION_MIXED && !yk;
   const size_t per_warp = mixed ? l2p_warp_bytes<P, float, false>(P_.cache->ld)
                                 : (yk ? l2p_warp_bytes<P, double, true>(P_.cache->ld) : l2p_warp_bytes<P, double, false>(P_.cache->ld));
-  const int warps = per_warp > 8192 ? 4 : 8;
-  const size_t smem = per_warp * warps;
+  // a CTA of four warps a leaf while there are no more than eight leaves an SM, which would leave its warp
+  // schedulers idle (a sphere of 31,000 points p = 16: near field and L2P 0.276 → 0.233 ms; Yukawa 40,000
+  // points p = 16, the whole pass 1.13 → 1.04); with more, a warp a leaf prepares its own entries without
+  // waiting for others
+  const int team = ng <= 8 * P_.ctx->num_sms;
+  const int warps = team || per_warp > 8192 ? 4 : 8;
+  const size_t smem = per_warp * (team ? 1 : warps);
   auto kern = mixed ? k_l2p<P, float, false> : (yk ? k_l2p<P, double, true> : k_l2p<P, double, false>);
   FMMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  kern<<<(ng + warps - 1) / warps, 32 * warps, smem, P_.ctx->stream>>>(gnode, gstart, gcount, ng, tx, ty, tz, tout, P_.cell.p,
-                                                                      S.Pl.p, P_.cache->ld, geometry(P_), P_.d_scale.p,
-                                                                      outputs, pot, grad, P_.d_kh2.p, acc);
+  kern<<<team ? ng : (ng + warps - 1) / warps, 32 * warps, smem, P_.ctx->stream>>>(
+      gnode, gstart, gcount, ng, tx, ty, tz, tout, P_.cell.p, S.Pl.p, P_.cache->ld, geometry(P_), P_.d_scale.p, outputs, pot,
+      grad, P_.d_kh2.p, acc, team);
   FMMB_LAUNCH_CHECK();
 }
 

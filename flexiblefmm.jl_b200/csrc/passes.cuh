@@ -42,6 +42,45 @@ template <typename R> __device__ __forceinline__ R ce(int i);
 template <> __device__ __forceinline__ double ce<double>(int i) { return c_e[i]; }
 template <> __device__ __forceinline__ float ce<float>(int i) { return c_ef[i]; }
 
+// An entry (m, n), the q-th m-major, of a local expansion prepared for L2P (harmonics.jl:447-486): the
+// potential's coefficient pair and the three gradient components' pairs (each from the degree-(n+1)
+// coefficients and the recurrence tables), the factor 2 of the m ≥ 1 terms folded in, so that every term of
+// the point loop is a complex dot product a·v with the regular harmonic v = Υ̃_n^m(x̂)
+template <int P>
+__host__ __device__ constexpr int l2p_entries() { return (P + 1) * (P + 2) / 2; }
+__device__ __forceinline__ int l2p_entry(int P, int m, int n) { return m * (P + 1) - m * (m - 1) / 2 + n - m; }
+template <int P>
+__device__ __forceinline__ void l2p_values(const double* __restrict__ L, int q, double (&v)[8]) {
+  int m = 0, rem = q;
+  while (rem >= P + 1 - m) { rem -= P + 1 - m; ++m; }
+  const int n = m + rem;
+  for (int i = 0; i < 8; ++i) v[i] = 0.0;
+  // potential: Σ L_n^m conj Υ̃ (harmonics.jl:455-462)
+  if (m == 0) v[0] = L[n * n];
+  else { v[0] = 2 * L[n * n + 2 * m - 1]; v[1] = 2 * L[n * n + 2 * m]; }
+  // gradient from degree n + 1 (harmonics.jl:465-486)
+  if (n < P) {
+    const int n1 = n + 1;
+    if (m == 0) {
+      const double cmv = ctab<double>(3 * TRI_MAX + tri(n1, 1));
+      v[2] = -cmv * L[n1 * n1 + 1];
+      v[4] = -cmv * L[n1 * n1 + 2];
+      v[6] = ctab<double>(2 * TRI_MAX + tri(n1, 0)) * L[n1 * n1];
+    } else {
+      const double ur = L[n1 * n1 + 2 * (m + 1) - 1], ui = L[n1 * n1 + 2 * (m + 1)];
+      double dr, di;
+      if (m == 1) { dr = L[n1 * n1]; di = 0; }
+      else { dr = L[n1 * n1 + 2 * (m - 1) - 1]; di = L[n1 * n1 + 2 * (m - 1)]; }
+      const double cu = 0.5 * ctab<double>(3 * TRI_MAX + tri(n1, m + 1));
+      const double cd = 0.5 * ctab<double>(4 * TRI_MAX + tri(n1, m - 1));
+      const double czv = ctab<double>(2 * TRI_MAX + tri(n1, m));
+      v[2] = 2 * (-cu * ur + cd * dr); v[3] = 2 * (-cu * ui + cd * di);
+      v[4] = -2 * (cu * ui + cd * di); v[5] = 2 * (cu * ur + cd * dr);
+      v[6] = 2 * czv * L[n1 * n1 + 2 * m - 1]; v[7] = 2 * czv * L[n1 * n1 + 2 * m];
+    }
+  }
+}
+
 // L2P at x̂ (potential and the gradient before the 1/w factor) from the local L in shared
 // memory, in precision R (FP64 on the plain path, FP32 on the mixed path); the orders run as a
 // loop (a full unroll keeps too many coefficients in registers)
