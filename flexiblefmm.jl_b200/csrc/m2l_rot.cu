@@ -458,23 +458,42 @@ __global__ void __launch_bounds__(32 * NW * G, MINB) k_rot(const __grid_constant
       // scatter: a warp the runs w, w + NW, ..., the entries across the lanes; then the next chunk's
       // multipoles into the rows it has read
       const int nrun = L[4 * NC + 1];
-      for (int r = warp; r < nrun; r += NW) {
-        const int j0 = L[3 * NC + r], j1 = L[3 * NC + r + 1];
-        double* dst = Pc + (int64_t)L[2 * NC + j0] * pitch;
-        // a parent's multipole starts from zero: its eight children are one run
-        double v[NE];
+      if constexpr (MODE == ROT_M2M) {
+        // few runs (a parent's eight children are one): a warp a run's 32 entries at a time, and the next
+        // chunk's rows over all warps. A parent's multipole starts from zero.
+        for (int r = 0; r < nrun; ++r) {
+          const int j0 = L[3 * NC + r], j1 = L[3 * NC + r + 1];
+          double* dst = Pc + (int64_t)L[2 * NC + j0] * pitch;
 #pragma unroll
-        for (int k = 0; k < NE; ++k) v[k] = MODE != ROT_M2M && lane + 32 * k < NP ? dst[lane + 32 * k] : 0.0;
-        for (int j = j0; j < j1; ++j)
+          for (int k = 0; k < NE; ++k) {
+            if ((r * NE + k) % NW != warp || lane + 32 * k >= NP) continue;
+            double v = 0.0;
+            for (int j = j0; j < j1; ++j) v = fma(alpha, tile[j * PT + loc[k]], v);
+            dst[lane + 32 * k] = v;
+          }
+        }
+        if (nn > 0) {
+          gsync();
+          for (int j = warp; j < nn; j += NW) gather(Ln, j);
+        }
+      } else {
+        for (int r = warp; r < nrun; r += NW) {
+          const int j0 = L[3 * NC + r], j1 = L[3 * NC + r + 1];
+          double* dst = Pc + (int64_t)L[2 * NC + j0] * pitch;
+          double v[NE];
+#pragma unroll
+          for (int k = 0; k < NE; ++k) v[k] = lane + 32 * k < NP ? dst[lane + 32 * k] : 0.0;
+          for (int j = j0; j < j1; ++j)
+#pragma unroll
+            for (int k = 0; k < NE; ++k)
+              if (lane + 32 * k < NP) v[k] = fma(alpha, tile[j * PT + loc[k]], v[k]);
 #pragma unroll
           for (int k = 0; k < NE; ++k)
-            if (lane + 32 * k < NP) v[k] = fma(alpha, tile[j * PT + loc[k]], v[k]);
-#pragma unroll
-        for (int k = 0; k < NE; ++k)
-          if (lane + 32 * k < NP) dst[lane + 32 * k] = v[k];
-        if (nn > 0) {
-          __syncwarp();
-          for (int j = j0; j < min(j1, nn); ++j) gather(Ln, j);
+            if (lane + 32 * k < NP) dst[lane + 32 * k] = v[k];
+          if (nn > 0) {
+            __syncwarp();
+            for (int j = j0; j < min(j1, nn); ++j) gather(Ln, j);
+          }
         }
       }
       // rows past this chunk's last pair (a next chunk is longer only when this one is full)
