@@ -24,13 +24,14 @@
 // units): with a pair per lane each coefficient is a broadcast per 32 pairs and multiply-add (180
 // wavefronts a pair at p = 10, against 67 for the fragments, each of which serves NG groups), and the
 // blocks of 1 to p + 1 pad the 8 × 8 × 4 tiles by half, which costs less than it saves. Measured, M2L of a
-// uniform cloud (FMAs with a pair per lane → this): 400,000 points p = 10 5.98 → 5.42 ms, p = 14 12.5 →
-// 11.6, p = 16 19.8 → 16.5; 31,000 points on a sphere p = 16 0.66 → 0.61; p = 20 120,000 points 1.20 →
-// 1.24. The dense products before it: 9.4 ms at p = 10, 57 at p = 16. M2M and L2L (dense GEMMs → this):
+// uniform cloud (FMAs with a pair per lane → this): 400,000 points p = 10 5.98 → 5.23 ms, p = 14 12.5 →
+// 10.9, p = 16 19.8 → 15.2; 31,000 points on a sphere p = 16 0.66 → 0.55. The dense products before it:
+// 9.4 ms at p = 10, 57 at p = 16. M2M and L2L (dense GEMMs → this):
 // 0.146 → 0.071 and 0.103 → 0.083 ms at 400,000 points p = 10, 0.536 → 0.157 and 0.425 → 0.161 at p = 16.
 // Loading the next step's operands ahead within a product spilled (5.4 → 7.7 ms).
 #include <algorithm>
 #include <numeric>
+#include <type_traits>
 
 #include "d4h.cuh"
 #include "m2l_rot.h"
@@ -137,9 +138,10 @@ size_t rot_smem(const RotLayout& l, int NG, int G) {
 // offset's azimuth) instead of before it. The imaginary parts of multipoles are negated on the way in
 // (not in ROT_L2L, whose inputs are locals) and on the way out where the output is one (ROT_M2M):
 // Tᵐ then acts on the real and the imaginary parts alike.
-template <int MODE, int RT, int NG, bool BACK>
-__device__ __forceinline__ void rotate_degree(int l, int t, double* r, int PT, const double2* cs, int PM,
-                                              const double* __restrict__ B, const int (&down)[NG]) {
+template <int MODE, int P, int RT, int NG, bool BACK>
+__device__ __forceinline__ void rotate_degree(int l, int t, double* r, const double2* cs, const double* __restrict__ B,
+                                              const int (&down)[NG]) {
+  constexpr int PT = rot_row(P), PM = rot_cs(P);
   double ar[NG][RT][2], ai[NG][RT][2];
 #pragma unroll
   for (int q = 0; q < NG; ++q)
@@ -193,8 +195,9 @@ __device__ __forceinline__ void rotate_degree(int l, int t, double* r, int PT, c
 }
 
 // the translation of order m over the degrees m..p, in place
-template <int RT, int NG>
-__device__ __forceinline__ void translate_order(int m, int p, int t, double* r, int PT, const double* __restrict__ B) {
+template <int P, int RT, int NG>
+__device__ __forceinline__ void translate_order(int m, int t, double* r, const double* __restrict__ B) {
+  constexpr int p = P, PT = rot_row(P);
   double ar[NG][RT][2], ai[NG][RT][2];
 #pragma unroll
   for (int q = 0; q < NG; ++q)
@@ -235,19 +238,18 @@ __device__ __forceinline__ void translate_order(int m, int p, int t, double* r, 
     }
 }
 
-template <int MODE, int TMAX, int NG, bool BACK>
-__device__ __forceinline__ void rotate_any(int l, int t, double* r, int PT, const double2* cs, int PM, const double* B,
-                                           const int (&down)[NG]) {
-  if (l < 8) rotate_degree<MODE, 1, NG, BACK>(l, t, r, PT, cs, PM, B, down);
-  else if (TMAX < 3 || l < 16) rotate_degree<MODE, 2, NG, BACK>(l, t, r, PT, cs, PM, B, down);
-  else rotate_degree<MODE, TMAX < 3 ? 2 : 3, NG, BACK>(l, t, r, PT, cs, PM, B, down);
+template <int MODE, int P, int NG, bool BACK>
+__device__ __forceinline__ void rotate_any(int l, int t, double* r, const double2* cs, const double* B, const int (&down)[NG]) {
+  if (P < 8 || l < 8) rotate_degree<MODE, P, 1, NG, BACK>(l, t, r, cs, B, down);
+  else if (P < 16 || l < 16) rotate_degree<MODE, P, 2, NG, BACK>(l, t, r, cs, B, down);
+  else rotate_degree<MODE, P, 3, NG, BACK>(l, t, r, cs, B, down);
 }
-template <int TMAX, int NG>
-__device__ __forceinline__ void translate_any(int m, int p, int t, double* r, int PT, const double* B) {
-  const int s = p + 1 - m;
-  if (s <= 8) translate_order<1, NG>(m, p, t, r, PT, B);
-  else if (TMAX < 3 || s <= 16) translate_order<2, NG>(m, p, t, r, PT, B);
-  else translate_order<TMAX < 3 ? 2 : 3, NG>(m, p, t, r, PT, B);
+template <int P, int NG>
+__device__ __forceinline__ void translate_any(int m, int t, double* r, const double* B) {
+  const int s = P + 1 - m;
+  if (P < 8 || s <= 8) translate_order<P, 1, NG>(m, t, r, B);
+  else if (P < 16 || s <= 16) translate_order<P, 2, NG>(m, t, r, B);
+  else translate_order<P, 3, NG>(m, t, r, B);
 }
 
 __device__ __forceinline__ void cpa16(void* dst, const void* src) {
@@ -281,14 +283,17 @@ struct RotArgs {
   const double* trans;
 };
 
-// NG groups of 8 pairs per chunk, G groups of NW warps; TMAX: 8-output tiles of the largest block;
-// NE: 32-entry pieces of an expansion
-template <int MODE, int NG, int G, int NW, int TMAX, int NE, int MINB>
+// NG groups of 8 pairs per chunk, G groups of NW warps. The order is a template argument: with the tile's
+// pitches known the addresses are immediates (M2L, 400,000 points, the order an argument → this: p = 3
+// 2.25 → 1.88 ms, p = 6 3.34 → 2.95, p = 10 5.42 → 5.23, p = 16 16.5 → 15.2, p = 20 120,000 points 3.98 → 3.36:
+// of 460 instructions a pair and warp at p = 10 two thirds were integer).
+template <int MODE, int P, int NG, int G, int NW, int MINB>
 __global__ void __launch_bounds__(32 * NW * G, MINB) k_rot(const __grid_constant__ RotArgs A) {
   static_assert(MODE == ROT_M2L || G == 1, "one group of warps per CTA in the sweeps");
   const RotSched& sch = A.sch;
   constexpr int NC = 8 * NG, NT = 32 * NW, NL = rot_list(NC);
-  const int p = sch.lay.p, NP = (p + 1) * (p + 1), PT = rot_row(p), PM = rot_cs(p), nd = 32 * sch.lay.nd, nt = 32 * sch.lay.nt;
+  constexpr int p = P, NP = (P + 1) * (P + 1), NE = (NP + 31) / 32, PT = rot_row(P), PM = rot_cs(P);
+  const int nd = 32 * sch.lay.nd, nt = 32 * sch.lay.nt;
   const int tid = threadIdx.x % NT, grp = threadIdx.x / NT, warp = tid >> 5, lane = tid & 31;
   const int comp = blockIdx.y, psi = A.stokes && comp == 3, LD = A.LD;
   const int64_t pitch = A.pitch;
@@ -439,20 +444,20 @@ __global__ void __launch_bounds__(32 * NW * G, MINB) k_rot(const __grid_constant
 #pragma unroll 1
       for (int i = sch.first[0][warp]; i < sch.first[0][warp + 1]; ++i) {
         const int l = sch.order[0][i];
-        rotate_any<MODE, TMAX, NG, false>(l, t, row0, PT, cs_g, PM, D + 32 * sch.lay.offd[l] + lane, down);
+        rotate_any<MODE, P, NG, false>(l, t, row0, cs_g, D + 32 * sch.lay.offd[l] + lane, down);
       }
       if (warp == 0 && nn > 0) commit(Ln, nn, pr);
       gsync();
 #pragma unroll 1
       for (int i = sch.first[1][warp]; i < sch.first[1][warp + 1]; ++i) {
         const int m = sch.order[1][i];
-        translate_any<TMAX, NG>(m, p, t, row0, PT, T + 32 * sch.lay.offt[m] + lane);
+        translate_any<P, NG>(m, t, row0, T + 32 * sch.lay.offt[m] + lane);
       }
       gsync();
 #pragma unroll 1
       for (int i = sch.first[0][warp]; i < sch.first[0][warp + 1]; ++i) {
         const int l = sch.order[0][i];
-        rotate_any<MODE, TMAX, NG, true>(l, t, row0, PT, cs_g, PM, D + 32 * sch.lay.offd[l] + lane, down);
+        rotate_any<MODE, P, NG, true>(l, t, row0, cs_g, D + 32 * sch.lay.offd[l] + lane, down);
       }
       gsync();
       // scatter: a warp the runs w, w + NW, ..., the entries across the lanes; then the next chunk's
@@ -503,6 +508,17 @@ __global__ void __launch_bounds__(32 * NW * G, MINB) k_rot(const __grid_constant
   }
 }
 
+// f(std::integral_constant<int, p>)
+template <class F>
+void for_order(int p, F&& f) {
+  switch (p) {
+#define X(pp) case pp: f(std::integral_constant<int, pp>()); break;
+    FMMB_P_CASES(X)
+#undef X
+    default: throw Error(FMMB_ERR_UNSUPPORTED, "p out of range");
+  }
+}
+
 RotSched schedule(const RotLayout& lay, int nw) {
   RotSched s{};
   s.lay = lay;
@@ -549,11 +565,11 @@ int parts_per_block(const Plan& P, int nexp, int slots, int nc) {
   return best;
 }
 
-template <int MODE, int NG, int G, int NW, int TMAX, int NE, int MINB>
+template <int MODE, int P, int NG, int G, int NW, int MINB>
 void start(RotArgs& A, const RotHost& R, int ctas, int nexp, cudaStream_t s) {
   A.sch = schedule(R.layout, NW);
   const size_t smem = rot_smem(R.layout, NG, G);
-  auto kern = k_rot<MODE, NG, G, NW, TMAX, NE, MINB>;
+  auto kern = k_rot<MODE, P, NG, G, NW, MINB>;
   FMMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<dim3(ctas, nexp), 32 * NW * G, smem, s>>>(A);
   FMMB_LAUNCH_CHECK();
@@ -572,7 +588,7 @@ RotArgs common_args(State& S, const double* cst, const double* in, double* out) 
   return A;
 }
 
-template <int NG, int G, int NW, int TMAX, int NE, int MINB>
+template <int ORD, int NG, int G, int NW, int MINB>
 void launch(State& S) {
   Plan& P = *S.plan;
   Cache& K = *P.cache;
@@ -588,11 +604,11 @@ void launch(State& S) {
   A.pairs = P.pairs.p;
   A.lv_trans = P.d_lv_rot.p;
   A.m2l_scale = P.d_m2l_scale.p;
-  start<ROT_M2L, NG, G, NW, TMAX, NE, MINB>(A, *K.rot, (A.nparts + G - 1) / G, K.nexp, P.ctx->stream);
+  start<ROT_M2L, ORD, NG, G, NW, MINB>(A, *K.rot, (A.nparts + G - 1) / G, K.nexp, P.ctx->stream);
 }
 
 // the children of level l (into their parents, or from them): chunks spread over the CTAs that run at once
-template <int MODE, int NG, int NW, int TMAX, int NE, int MINB>
+template <int MODE, int ORD, int NG, int NW, int MINB>
 void launch_sweep(State& S, int l, const double* trans) {
   Plan& P = *S.plan;
   Cache& K = *P.cache;
@@ -603,16 +619,16 @@ void launch_sweep(State& S, int l, const double* trans) {
   A.trans = trans;
   const int slots = std::max(1, P.ctx->num_sms * MINB / K.nexp), chunks = (A.nchild + 8 * NG - 1) / (8 * NG);
   A.per = 8 * NG * ((chunks + slots - 1) / slots);
-  start<MODE, NG, 1, NW, TMAX, NE, MINB>(A, *K.rot, (A.nchild + A.per - 1) / A.per, K.nexp, P.ctx->stream);
+  start<MODE, ORD, NG, 1, NW, MINB>(A, *K.rot, (A.nchild + A.per - 1) / A.per, K.nexp, P.ctx->stream);
 }
 
 template <int MODE>
 void sweep(State& S, int l, const double* trans) {
-  const int p = S.plan->cache->p;
-  if (p <= 11) launch_sweep<MODE, 3, 4, 2, 5, 4>(S, l, trans);
-  else if (p <= 15) launch_sweep<MODE, 3, 6, 2, 8, 2>(S, l, trans);
-  else if (p == 16) launch_sweep<MODE, 2, 8, 3, 10, 1>(S, l, trans);
-  else launch_sweep<MODE, 2, 8, 3, 14, 1>(S, l, trans);
+  auto go = [&](auto order) {
+    constexpr int P = decltype(order)::value;
+    launch_sweep<MODE, P, P <= 15 ? 3 : 2, P <= 11 ? 4 : (P <= 15 ? 6 : 8), P <= 11 ? 4 : (P <= 15 ? 2 : 1)>(S, l, trans);
+  };
+  for_order(S.plan->cache->p, go);
 }
 
 // the translations along z of n classes (c0 ..) from their dense operators
@@ -688,19 +704,22 @@ void prepare_rotations(Plan& P) {
 void m2m_rot(State& S, int l) { sweep<ROT_M2M>(S, l + 1, S.plan->lv_rot_m2m[l]); }
 void l2l_rot(State& S, int l) { sweep<ROT_L2L>(S, l, S.plan->lv_rot_l2l[l - 1]); }
 
-// Chunks of 24 pairs and two to four CTAs per SM while the tiles and tables fit (400,000 points p = 10:
+// (Measured with the order an argument.) Chunks of 24 pairs and two to four CTAs per SM while the tiles
+// and tables fit (400,000 points p = 10:
 // 5.42 ms, sphere of 30,000 0.49; chunks of 16 6.42 and 0.50; two groups with chunks of 32 5.50 and 0.65.
 // p = 14: 11.6; chunks of 16 14.4; four warps instead of six 13.8). At p = 16 one CTA fits: two groups of
 // warps share the rotations, one computing while the other scatters, as long as there are pairs enough
 // for that many chunks (6.04M pairs: 16.5 ms against 23.8 for one group; 1.05M: 3.83 against 4.31), one
 // group where there are not (71,365: 0.61 against 0.64; 56,448: 0.46 against 0.64).
 void m2l_rot(State& S) {
-  const int p = S.plan->cache->p;
-  if (p <= 11) launch<3, 1, 4, 2, 5, 4>(S);
-  else if (p <= 15) launch<3, 1, 6, 2, 8, 2>(S);
-  else if (p == 16 && (int64_t)S.plan->npairs * S.plan->cache->nexp >= 1000000) launch<3, 2, 6, 3, 10, 1>(S);
-  else if (p == 16) launch<2, 1, 8, 3, 10, 1>(S);
-  else launch<2, 1, 8, 3, 14, 1>(S);
+  const bool many = (int64_t)S.plan->npairs * S.plan->cache->nexp >= 1000000;
+  for_order(S.plan->cache->p, [&](auto order) {
+    constexpr int P = decltype(order)::value;
+    if constexpr (P <= 11) launch<P, 3, 1, 4, 4>(S);
+    else if constexpr (P <= 15) launch<P, 3, 1, 6, 2>(S);
+    else if (P == 16 && many) launch<16, 3, 2, 6, 1>(S);
+    else launch<P, 2, 1, 8, 1>(S);
+  });
 }
 
 }  // namespace fmmb
