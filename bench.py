@@ -621,9 +621,8 @@ def run_ours(a):
         f = fmmb.FMM(m, pts, ppl=a.ppl, bbox=((0.0, 0.0, 0.0), 1.0))
         plan_s = time.perf_counter() - t0
         states = {"mixed": fmmb.FMMState(f, "mixed"), "fp64": fmmb.FMMState(f, "fp64")}
-        # the launch shapes tuned on these inputs (fmmb_autotune; no result depends on them): the
-        # FP64 path's chunk width and near-field warps, then the mixed path's, with the plan's M2L
-        # block size, which both paths share
+        # the launch shape tuned on these inputs (fmmb_autotune; no result depends on it): the plan's
+        # M2L block size, which both paths share, on the mixed path; the FP64 path's stages timed
         tuned = {"fp64": fmmb.autotune(states["fp64"], pts, tau, tune_blocks=False),
                  "mixed": fmmb.autotune(states["mixed"], pts, tau, tune_blocks=True)}
 

@@ -20,10 +20,11 @@
 //              the sums depend neither on where the chunks end nor on the other targets); the warp then
 //              sends the next chunk's inputs (cp.async) into the rows it has read
 // The products run on the FP64 tensor cores, 8 pairs × 4 inputs as A and the coefficients as B, laid out
-// in fragments on the host. What bounds the kernel is shared memory, not the FP64 rate (equal on the FMA
-// units): with a pair per lane each coefficient is a broadcast per 32 pairs and multiply-add (180
-// wavefronts a pair at p = 10, against 67 for the fragments, each of which serves NG groups), and the
-// blocks of 1 to p + 1 pad the 8 × 8 × 4 tiles by half, which costs less than it saves. Measured, M2L of a
+// in fragments on the host; a fragment serves the NG groups of a chunk, where FMAs with a pair per lane read a
+// coefficient per multiply-add (180 shared-memory wavefronts a pair at p = 10). The blocks of 1 to p + 1 pad the
+// 8 × 8 × 4 tiles by half, which costs less than it saves. What bounds the kernel is the L1 / shared-memory pipe
+// (two thirds busy: the tile is read and written three times) and instruction issue, not the FP64 rate (equal on
+// the FMA units). Measured, M2L of a
 // uniform cloud (FMAs with a pair per lane → this): 400,000 points p = 10 5.98 → 5.23 ms, p = 14 12.5 →
 // 10.9, p = 16 19.8 → 15.2; 31,000 points on a sphere p = 16 0.66 → 0.55. The dense products before it:
 // 9.4 ms at p = 10, 57 at p = 16. M2M and L2L (dense GEMMs → this):

@@ -182,8 +182,8 @@ function build_expansions!(st::FMMState, f::FMM, sources::AbstractVector{SVector
     return st
 end
 # The launch shapes of this state timed on its own inputs and the fastest kept (fmmb_autotune);
-# no result depends on them. Returns (block targets, FP64 chunk variant, near-field warps,
-# M2L ms, near-field ms).
+# no result depends on them. Returns (block targets, 0, 4, M2L ms, near-field ms); the second and
+# third (FP64 chunk variant, near-field warps) are no longer chosen.
 function autotune!(st::FMMState, f::FMM, sources::AbstractVector{SVector{3,Float64}}, τ::AbstractVector{<:Real};
                    tune_blocks::Bool=true)
     length(sources) == f.n || throw(DimensionMismatch("expected $(f.n) sources"))
