@@ -98,7 +98,7 @@ __global__ void k_stokes_q4(const int* __restrict__ nodes, int nn, const int4* _
 // memory, NV coefficient pairs each (Φ_i + ∂̂_iΨ̂, then ∂̂_iΦ_k at 3 + 3i + k; PRES: the divergence), then a
 // warp 32 targets at a time runs the recurrence once for all of them. Bound by the entries' shared-memory
 // reads. Measured (four unprepared L2Ps per target, a warp a leaf → this): 13,704 leaves of twelve spheres p = 16
-// 3.06 → 1.34 ms; 332 leaves with densities p = 12 the whole call 2.50 → 1.72.
+// 3.06 → 1.34 ms; 332 leaves and 395 of targets p = 12 0.84 → 0.072 (the whole call with densities 2.50 → 1.72).
 template <int P, bool PRES>
 __global__ void __launch_bounds__(SW * 32) k_stokes_l2p(const int* __restrict__ gnode, const int* __restrict__ gstart,
                                                         const int* __restrict__ gcount, const double* __restrict__ tx,
