@@ -39,7 +39,5 @@ struct RotHost {
 };
 
 std::shared_ptr<const RotHost> rotation_tables(int p, const HostOperators& op);
-// the Gauss–Legendre rule on [−1, 1] of n points
-void gauss_legendre(int n, std::vector<double>& t, std::vector<double>& w);
 
 }  // namespace fmmb

@@ -20,7 +20,6 @@
 #include <map>
 #include <tuple>
 
-#include "m2l_rot.h"
 #include "passes.cuh"
 
 namespace fmmb {
@@ -148,6 +147,38 @@ __global__ void k_yk_projection(int p, int LD, int nq, const double* __restrict_
     }
   }
   for (int i = (p + 1) * (p + 1); i < LD; ++i) col[i] = 0;
+}
+
+// the Gauss–Legendre rule on [−1, 1] of n points by Newton's iteration on P_n (the reference
+// takes the Golub–Welsch eigenvalues, harmonics_yukawa.jl:89-93: the same rule to rounding)
+void gauss_legendre(int n, std::vector<double>& t, std::vector<double>& w) {
+  t.assign(n, 0.0);
+  w.assign(n, 0.0);
+  for (int i = 0; i < (n + 1) / 2; ++i) {
+    double x = std::cos(M_PI * (i + 0.75) / (n + 0.5)), dp = 0;
+    for (int it = 0; it < 100; ++it) {
+      double p0 = 1, p1 = x;
+      for (int k = 2; k <= n; ++k) {
+        const double p2 = ((2 * k - 1) * x * p1 - (k - 1) * p0) / k;
+        p0 = p1;
+        p1 = p2;
+      }
+      dp = n * (x * p1 - p0) / (x * x - 1);
+      const double dx = p1 / dp;
+      x -= dx;
+      if (std::fabs(dx) < 1e-16) break;
+    }
+    double p0 = 1, p1 = x;
+    for (int k = 2; k <= n; ++k) {
+      const double p2 = ((2 * k - 1) * x * p1 - (k - 1) * p0) / k;
+      p0 = p1;
+      p1 = p2;
+    }
+    dp = n * (x * p1 - p0) / (x * x - 1);
+    t[i] = -x;
+    t[n - 1 - i] = x;
+    w[i] = w[n - 1 - i] = 2 / ((1 - x * x) * dp * dp);
+  }
 }
 
 // the product rule on the unit sphere (harmonics_yukawa.jl:94-110), uploaded once per cache
