@@ -68,21 +68,20 @@ enum : int { ROT_M2L = 0, ROT_M2M = 1, ROT_L2L = 2 };
 
 // T of class c0 + blockIdx.x from its dense operator A (column-major, lda; stride per class):
 // T^m_{ll'} = the (Re l m, Re l' m) entry of D A D⁻¹, negated for odd m on both sides' behalf (Σ
-// above): a thread per entry. Multipoles transform by the conjugate of the locals' rotation.
+// above): a CTA per class and input degree l' = blockIdx.y, a thread per entry; T is zeroed by the caller.
+// (M2M and L2L are one class each: with a CTA per class alone the first state of a cache took 1.5 ms at p = 16
+// and 3.8 at p = 20, now 0.65 and 1.2.) Multipoles transform by the conjugate of the locals' rotation.
 __global__ void k_rot_translations(const double* __restrict__ dense, int lda, int64_t stride, int mode, int c0,
                                    const double* __restrict__ dtab, const double* __restrict__ cstab, RotLayout lay,
                                    double* __restrict__ out) {
-  const int p = lay.p, c = c0 + blockIdx.x;
+  const int p = lay.p, c = c0 + blockIdx.x, l2 = blockIdx.y;
   const double* A = dense + blockIdx.x * stride;
   const double sin_in = mode == ROT_L2L ? 1.0 : -1.0, sin_out = mode == ROT_M2M ? -1.0 : 1.0;
   const double* d = dtab + (int64_t)c * 32 * lay.nd;
   const double* cs = cstab + (int64_t)c * 2 * (p + 1);
   double* T = out + (int64_t)blockIdx.x * 32 * lay.nt;
-  for (int i = threadIdx.x; i < 32 * lay.nt; i += blockDim.x) T[i] = 0.0;
-  __syncthreads();
-  const int np = (p + 1) * (p + 1) * (p + 1);
-  for (int i = threadIdx.x; i < np; i += blockDim.x) {
-    const int m = i % (p + 1), l = i / (p + 1) % (p + 1), l2 = i / ((p + 1) * (p + 1));
+  for (int i = threadIdx.x; i < (p + 1) * (p + 1); i += blockDim.x) {
+    const int m = i % (p + 1), l = i / (p + 1);
     if (m > l || m > l2) continue;
     double sum = 0;
     for (int b = 0; b <= l2; ++b) {
@@ -636,7 +635,8 @@ void sweep(State& S, int l, const double* trans) {
 void translations(Cache& C, const RotLayout& lay, int mode, int c0, int n, const double* dense, int lda, int64_t stride,
                   DBuf<double>& out, cudaStream_t s) {
   out.alloc((size_t)n * 32 * lay.nt);
-  k_rot_translations<<<n, 256, 0, s>>>(dense, lda, stride, mode, c0, C.rot_d.p, C.rot_cs.p, lay, out.p);
+  FMMB_CUDA(cudaMemsetAsync(out.p, 0, out.bytes(), s));
+  k_rot_translations<<<dim3(n, lay.p + 1), 128, 0, s>>>(dense, lda, stride, mode, c0, C.rot_d.p, C.rot_cs.p, lay, out.p);
   FMMB_LAUNCH_CHECK();
 }
 void all_translations(Cache& C, const RotLayout& lay, const double* reps, const double* m2m, const double* l2l,
