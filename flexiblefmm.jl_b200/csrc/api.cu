@@ -758,7 +758,7 @@ int fmmb_build_expansions(fmmb_state* state, const double* xyz, const double* ta
     require(n == P.N, FMMB_ERR_DIMENSION, "expected " + std::to_string(P.N) + " sources and densities");
     set_device(*P.ctx);
     cudaStream_t s = P.ctx->stream;
-    if (S.h_in_xyz.n < (size_t)(3 * n)) { S.h_in_xyz.alloc(3 * n); S.h_in_tau.alloc(n); }
+    if (S.h_in_tau.n < (size_t)n) { S.h_in_xyz.alloc(3 * n); S.h_in_tau.alloc(n); }
     FMMB_CUDA(cudaMemcpyAsync(S.h_in_xyz.p, xyz, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
     FMMB_CUDA(cudaMemcpyAsync(S.h_in_tau.p, tau, sizeof(double) * n, cudaMemcpyHostToDevice, s));
     state_build(S, S.h_in_xyz.p, S.h_in_tau.p);
@@ -831,7 +831,7 @@ int fmmb_evaluate_at_sources(fmmb_state* state, int outputs, double* pot, double
     require(!(outputs & FMMB_OUTPUT_GRADIENT) || grad, FMMB_ERR_ARGUMENT, "null gradient output");
     set_device(*P.ctx);
     cudaStream_t s = P.ctx->stream;
-    if (S.d_pot.n < (size_t)P.N) { S.d_pot.alloc(P.N); S.d_grad.alloc(3 * P.N); }
+    if (S.d_grad.n < (size_t)(3 * P.N)) { S.d_pot.alloc(P.N); S.d_grad.alloc(3 * P.N); }
     evaluate_sources(S, outputs, S.d_pot.p, S.d_grad.p);
     if (outputs & FMMB_OUTPUT_POTENTIAL)
       FMMB_CUDA(cudaMemcpyAsync(pot, S.d_pot.p, sizeof(double) * P.N, cudaMemcpyDeviceToHost, s));
@@ -885,8 +885,8 @@ int fmmb_matvec(fmmb_state* state, const double* xyz, const double* tau, int64_t
     require(!(outputs & FMMB_OUTPUT_GRADIENT) || grad, FMMB_ERR_ARGUMENT, "null gradient output");
     set_device(*P.ctx);
     cudaStream_t s = P.ctx->stream;
-    if (S.h_in_xyz.n < (size_t)(3 * n)) { S.h_in_xyz.alloc(3 * n); S.h_in_tau.alloc(n); }
-    if (S.d_pot.n < (size_t)P.N) { S.d_pot.alloc(P.N); S.d_grad.alloc(3 * P.N); }
+    if (S.h_in_tau.n < (size_t)n) { S.h_in_xyz.alloc(3 * n); S.h_in_tau.alloc(n); }
+    if (S.d_grad.n < (size_t)(3 * P.N)) { S.d_pot.alloc(P.N); S.d_grad.alloc(3 * P.N); }
     FMMB_CUDA(cudaMemcpyAsync(S.h_in_xyz.p, xyz, sizeof(double) * 3 * n, cudaMemcpyHostToDevice, s));
     FMMB_CUDA(cudaMemcpyAsync(S.h_in_tau.p, tau, sizeof(double) * n, cudaMemcpyHostToDevice, s));
     matvec_sources(S, S.h_in_xyz.p, S.h_in_tau.p, outputs, S.d_pot.p, S.d_grad.p);

@@ -54,22 +54,25 @@ struct DBuf {
     return *this;
   }
   ~DBuf() { release(); }
-  static void raw_alloc(T** q, size_t count, cudaStream_t st) {
-    if (st) FMMB_CUDA(cudaMallocAsync((void**)q, count * sizeof(T), st));
-    else FMMB_CUDA(cudaMalloc((void**)q, count * sizeof(T)));
+  static T* raw_alloc(size_t count, cudaStream_t st) {
+    void* q = nullptr;
+    if (st) FMMB_CUDA(cudaMallocAsync(&q, count * sizeof(T), st));
+    else FMMB_CUDA(cudaMalloc(&q, count * sizeof(T)));
+    return (T*)q;
   }
+  // empty when the allocation fails: n entries are always there (of buffers that grow together, callers ask
+  // the one allocated last)
   void alloc(size_t count) {
     release();
-    n = count;
     s = g_alloc_stream;
-    if (count) raw_alloc(&p, count, s);
+    if (count) p = raw_alloc(count, s);
+    n = count;
   }
   // grow to at least `count` entries, keeping the first `keep`
   void grow(size_t count, size_t keep, cudaStream_t st) {
     if (count <= n) return;
     size_t cap = std::max(count, n * 2);
-    T* q = nullptr;
-    raw_alloc(&q, cap, g_alloc_stream);
+    T* q = raw_alloc(cap, g_alloc_stream);
     if (keep && p) FMMB_CUDA(cudaMemcpyAsync(q, p, keep * sizeof(T), cudaMemcpyDeviceToDevice, st));
     FMMB_CUDA(cudaStreamSynchronize(st));
     release();

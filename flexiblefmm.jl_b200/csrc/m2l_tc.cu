@@ -841,10 +841,10 @@ void m2l_mixed(State& S) {
   if (nb == 0) return;
   const int KP = kp_of(C.np);
   const size_t ne = (size_t)P.nnodes * KP;
-  if (S.Mh.n < 2 * ne) { S.Mh.alloc(2 * ne); S.Ml.alloc(2 * ne); }
+  if (S.Ml.n < 2 * ne) { S.Mh.alloc(2 * ne); S.Ml.alloc(2 * ne); }
   const int nseg = P.nseg;                         // one scale per segment (per level for one point set)
   const int* seg = P.ninst > 1 ? P.node_seg.p : nullptr;
-  if (S.Lsc.n < (size_t)nseg) { S.Lsc.alloc(nseg); S.Lmax.alloc(nseg); }
+  if (S.Lmax.n < (size_t)nseg) { S.Lsc.alloc(nseg); S.Lmax.alloc(nseg); }
   if (!S.err.p) {                                  // sticky until reported (mixed_error_flag clears it)
     S.err.alloc(1);
     FMMB_CUDA(cudaMemsetAsync(S.err.p, 0, sizeof(int), s));

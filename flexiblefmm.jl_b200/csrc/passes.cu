@@ -533,7 +533,8 @@ int group_targets(State& S, const double* tg, int64_t nt) {
   cudaStream_t s = P.ctx->stream;
   require(P.ninst == 1, FMMB_ERR_UNSUPPORTED, "a batch plan evaluates at its sources only");
   require(nt < (1ll << 31) - 1, FMMB_ERR_ARGUMENT, "too many targets");
-  if ((int64_t)S.t_x.n < nt) {
+  if ((int64_t)S.t_groups.n < 3 * nt + 3) {
+    S.t_groups.release();                        // the last: too short until all are there
     S.t_x.alloc(nt); S.t_y.alloc(nt); S.t_z.alloc(nt); S.t_out.alloc(nt); S.t_node.alloc(nt);
     S.t_keys.alloc(nt); S.t_vals.alloc(nt); S.t_groups.alloc(3 * nt + 3);
   }
