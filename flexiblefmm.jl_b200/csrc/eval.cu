@@ -210,7 +210,7 @@ struct ChargesNear {
         acc[0] = fma(-sv.w, self ? 0.0 : log(r2), acc[0]);
         if (GRAD) qir3 = self ? 0.0 : 2 * sv.w / r2;
       } else {
-        double ir = rsqrt_h(r2), w = sv.w;
+        double ir = rsqrt(r2), w = sv.w;
         if (CHECK && i == is) ir = 0.0;
         if constexpr (KERNEL == 1) {
           const double kr = __dmul_rn(pa.kappa, __dmul_rn(r2, ir));
@@ -483,7 +483,7 @@ struct DipolesNear {
       const R vx = t[0] - sv.x, vy = t[1] - sv.y, vz = t[2] - sv.z;
       const R r2 = vx * vx + vy * vy + vz * vz;
       R ir;
-      if constexpr (sizeof(R) == 8) ir = r2 > 0.0 ? rsqrt_h(r2) : 0.0;
+      if constexpr (sizeof(R) == 8) ir = r2 > 0.0 ? rsqrt(r2) : 0.0;
       else ir = r2 > 0.f ? 1.f / sqrtf(r2) : 0.f;
       if (CHECK && i == is) ir = R(0);
       const R ir2 = ir * ir, ir3 = ir2 * ir;

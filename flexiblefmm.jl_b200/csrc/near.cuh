@@ -28,18 +28,6 @@ namespace {
 
 constexpr int NEAR_TEAM = 4, NEAR_ALONE = 10000;
 
-// 1/√x in FP64: the hardware's coarse value y (PTX rsqrt.approx.ftz.f64) and one third-order
-// Householder step y(1 + e(½ + ⅜e)), e = 1 − xy², whose error is (5/16)e³, far below one rounding.
-// Five FMAs where the library's call takes about twice that; zero, tiny, huge and non-finite arguments
-// go to the library's.
-__device__ __forceinline__ double rsqrt_h(double x) {
-  double y;
-  asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double e = fma(-(x * y), y, 1.0);
-  const double r = fma(y * e, fma(0.375, e, 0.5), y);
-  return (unsigned)__double2hiint(x) - 0x03000000u < 0x79000000u ? r : rsqrt(x);
-}
-
 // the targets' groups (per leaf: node, first target, count), the targets in group order and their
 // output indices, and the tree
 struct NearArgs {

@@ -308,7 +308,7 @@ struct StokesNear {
       const SV sv = st.s[i];
       const double dx = t[0] - sv.x, dy = t[1] - sv.y, dz = t[2] - sv.z;
       const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
-      double ir = rsqrt_h(r2);
+      double ir = rsqrt(r2);
       if (CHECK && i == is) ir = 0.0;
       const double ir3 = ir * ir * ir;
       const double df = dx * sv.fx + dy * sv.fy + dz * sv.fz;
