@@ -452,12 +452,16 @@ __global__ void __launch_bounds__(128) k_kic_l2t(const int* __restrict__ gnode, 
 // src/sources.jl:137-155 with Laplace3D): per source q/r + (d·v)/r³ and the gradient
 // −q v/r³ + d/r³ − 3 v (d·v)/r⁵, v = t − s, as KC times the sums below (pot += KC·Σ, grad −= KC·Σ);
 // coincident points contribute nothing. R = float: relative to the leaf's centre, batches summed in
-// FP32 and their sums in FP64.
+// FP32 and their sums in FP64; the reciprocal root correctly rounded, in one step: as 1/√r², in a division and a
+// root, it bounded the kernel at this frame's occupancy (500,000 points, 2·10⁶ targets p = 4, the whole evaluation: a
+// warp a leaf 3.05 ms, this frame with the division 5.17, with __frsqrt_rn 2.70, five CTAs an SM and four
+// sources at a time 2.42; 60,000 points at the sources p = 11 0.198, 0.225, 0.201, 0.192). FP64, 500,000 points and
+// targets p = 4: two sources at a time 1.34, four 1.14, with selects 1.05 (a warp a leaf 1.89).
 template <typename R>
 struct DipolesNear {
   using Real = R;
   static constexpr bool REL = sizeof(R) == 4;
-  static constexpr int NA = 4, CH = 2, MINB = 4;
+  static constexpr int NA = 4, CH = 2, MINB = REL ? 5 : 4;
   struct Args {
     const double *xs, *ys, *zs, *q, *d3;
     int64_t npts;
@@ -477,15 +481,15 @@ struct DipolesNear {
   static __device__ __forceinline__ void batch(const Args&, const Stage& st, int m, int is, int part, int f, const R (&t)[3],
                                                double (&acc)[NA]) {
     R bp = 0, bx = 0, by = 0, bz = 0;
-#pragma unroll 2
+#pragma unroll 4
     for (int i = part; i < m; i += f) {
       const R4<R> sv = st.p[i], dv = st.d[i];
       const R vx = t[0] - sv.x, vy = t[1] - sv.y, vz = t[2] - sv.z;
       const R r2 = vx * vx + vy * vy + vz * vz;
       R ir;
-      if constexpr (sizeof(R) == 8) ir = r2 > 0.0 ? rsqrt(r2) : 0.0;
-      else ir = r2 > 0.f ? 1.f / sqrtf(r2) : 0.f;
-      if (CHECK && i == is) ir = R(0);
+      if constexpr (sizeof(R) == 8) ir = rsqrt(r2);
+      else ir = __frsqrt_rn(r2);
+      if (!(r2 > R(0)) || (CHECK && i == is)) ir = R(0);   // selects: a branch around the root cost a tenth of the time
       const R ir2 = ir * ir, ir3 = ir2 * ir;
       const R dd = dv.x * vx + dv.y * vy + dv.z * vz;
       bp += sv.w * ir + dd * ir3;
