@@ -68,3 +68,42 @@ def test_dipole_multipoles_match_charge_pairs(fmmb, p):
     assert f.nlevels == 3 and g.nnodes == f.nnodes
     P, _ = fmmb.build_expansions(g, two, q).expansions()
     assert mrd(P.ravel(), D.ravel()) < 1e-6
+
+
+SMALL = [1, 2, 4, 7, 8, 9, 12, 15, 16, 17]
+
+
+@pytest.mark.parametrize("p", [1, 2, 3, 4, 7, 8, 12, 15, 16])
+def test_small_nodes_match_oracle(oracle, fmmb, p):
+    """Nodes of at most 8 and 16 sources, which share a warp up to p = 15."""
+    rng = np.random.default_rng(740 + p)
+    pts = clumps(rng, SMALL)
+    tau = rng.standard_normal(len(pts))
+    O = oracle.FMM(p, pts, 20)
+    O.build_expansions(pts, tau)
+    OM, _ = O.expansions()
+    f = fmmb.FMM(fmmb.SphericalHarmonics(fmmb.Laplace3D(), p=p), pts, ppl=20, bbox=BOX)
+    M, _ = fmmb.build_expansions(f, pts, tau).expansions()
+    assert f.nlevels == 3 and M.shape == OM.shape and mrd(M.ravel(), OM.ravel()) < 1e-13
+
+
+@pytest.mark.parametrize("p,precision", [(1, "fp64"), (3, "mixed"), (6, "fp64"), (9, "mixed"), (15, "fp64"), (16, "fp64")])
+def test_small_nodes_same_in_a_large_launch(fmmb, p, precision):
+    """A list that fills the device gives each warp four nodes and each CTA all sets of its nodes (charges and the
+    dipoles' components); a node's sums depend on neither: a batch of eight instances, large, equals each
+    instance's own plan, small, bit by bit."""
+    rng = np.random.default_rng(760 + p)
+    m = fmmb.SphericalHarmonics(fmmb.Laplace3D(), p=p)
+    sets = [rng.random((30000, 3)) for _ in range(8)]
+    tau, mom = [rng.standard_normal(30000) for _ in sets], [0.1 * rng.standard_normal((30000, 3)) for _ in sets]
+    batch = fmmb.BatchFMM(m, sets, ppl=24, bbox=BOX)
+    cache = fmmb.OperatorCache(m)
+    alone = [fmmb.FMM(m, s, ppl=24, bbox=BOX, cache=cache) for s in sets[:2]]
+    assert alone[0].nnodes < 8000 and batch.nnodes > 32000
+    for dip in (False, True):
+        dens = lambda q, d: (q, fmmb.Dipoles(d)) if dip else q
+        u = fmmb.evaluate_at_sources(batch, fmmb.build_expansions(batch, batch.sources, dens(batch.concat(tau), np.concatenate(mom)),
+                                                                  precision=precision))
+        for i, f in enumerate(alone):
+            a = fmmb.evaluate_at_sources(f, fmmb.build_expansions(f, sets[i], dens(tau[i], mom[i]), precision=precision))
+            assert np.array_equal(batch.split(u)[i], a), (i, dip)
