@@ -117,21 +117,6 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
                : "d"(a), "d"(b));
 }
 
-// The tile's row of one pair: degree l from base(l) on, the l + 1 real parts of m = 0..l, then the l
-// imaginary parts; base(l) ≡ l (mod 4) and a row is an odd multiple of 4 doubles, so that the 8 pairs ×
-// 4 orders (or 4 degrees of one order) a warp reads or writes at once lie in distinct banks
-__host__ __device__ constexpr int rot_base(int l) { return l * l + 2 * (l / 2); }
-__host__ __device__ constexpr int rot_row(int p) { return (rot_base(p + 1) + 3) / 4 * 4 | 4; }
-// the row of the pair's (cos mφ, sin mφ): zeros past m = p for the padded inputs
-__host__ __device__ constexpr int rot_cs(int p) { return (p + 4) / 8 * 8 + 5; }
-constexpr int rot_list(int nc) { return 4 * nc + 2; }   // source, offset (bit 31: it points down), target, runs; the last run's end, their count
-
-size_t rot_smem(const RotLayout& l, int NG, int G) {
-  const int nc = 8 * NG;
-  return sizeof(double) * ((size_t)32 * (l.nd + G * l.nt) + (size_t)G * nc * (2 * rot_cs(l.p) + rot_row(l.p)) + 8) +
-         sizeof(int) * (size_t)G * 2 * rot_list(nc);
-}
-
 // the rotation of degree l of NG groups of 8 pairs, in place: r, cs: this lane's pair of the first
 // group (pair g), PT and PM apart per pair; B: the degree's fragments at this lane; down: per group
 // the sign bit where the pair's offset points down; BACK: the z rotation after the product (to the
@@ -289,6 +274,7 @@ struct RotArgs {
 // of 460 instructions a pair and warp at p = 10 two thirds were integer).
 template <int MODE, int P, int NG, int G, int NW, int MINB>
 __global__ void __launch_bounds__(32 * NW * G, MINB) k_rot(const __grid_constant__ RotArgs A) {
+  static_assert(MINB <= rot_resident(P, NG, G, MINB), "the CTAs that the launch counts on fit an SM");
   static_assert(MODE == ROT_M2L || G == 1, "one group of warps per CTA in the sweeps");
   const RotSched& sch = A.sch;
   constexpr int NC = 8 * NG, NT = 32 * NW, NL = rot_list(NC);
@@ -568,7 +554,7 @@ int parts_per_block(const Plan& P, int nexp, int slots, int nc) {
 template <int MODE, int P, int NG, int G, int NW, int MINB>
 void start(RotArgs& A, const RotHost& R, int ctas, int nexp, cudaStream_t s) {
   A.sch = schedule(R.layout, NW);
-  const size_t smem = rot_smem(R.layout, NG, G);
+  const size_t smem = rot_smem(P, NG, G);
   auto kern = k_rot<MODE, P, NG, G, NW, MINB>;
   FMMB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   kern<<<dim3(ctas, nexp), 32 * NW * G, smem, s>>>(A);
@@ -625,8 +611,8 @@ void launch_sweep(State& S, int l, const double* trans) {
 template <int MODE>
 void sweep(State& S, int l, const double* trans) {
   auto go = [&](auto order) {
-    constexpr int P = decltype(order)::value;
-    launch_sweep<MODE, P, P <= 15 ? 3 : 2, P <= 11 ? 4 : (P <= 15 ? 6 : 8), P <= 11 ? 4 : (P <= 15 ? 2 : 1)>(S, l, trans);
+    constexpr int P = decltype(order)::value, NG = P <= 15 ? 3 : 2;
+    launch_sweep<MODE, P, NG, P <= 11 ? 4 : (P <= 15 ? 6 : 8), rot_resident(P, NG, 1, P <= 11 ? 4 : (P <= 15 ? 2 : 1))>(S, l, trans);
   };
   for_order(S.plan->cache->p, go);
 }
@@ -708,16 +694,18 @@ void l2l_rot(State& S, int l) { sweep<ROT_L2L>(S, l, S.plan->lv_rot_l2l[l - 1]);
 // (Measured with the order an argument.) Chunks of 24 pairs and two to four CTAs per SM while the tiles
 // and tables fit (400,000 points p = 10:
 // 5.42 ms, sphere of 30,000 0.49; chunks of 16 6.42 and 0.50; two groups with chunks of 32 5.50 and 0.65.
-// p = 14: 11.6; chunks of 16 14.4; four warps instead of six 13.8). At p = 16 one CTA fits: two groups of
-// warps share the rotations, one computing while the other scatters, as long as there are pairs enough
-// for that many chunks (6.04M pairs: 16.5 ms against 23.8 for one group; 1.05M: 3.83 against 4.31), one
+// p = 14: 11.6; chunks of 16 14.4; four warps instead of six 13.8). Three CTAs fit at p = 11 (400,000 points: 8.33 ms, 8.49
+// with the registers and parts of four; M2M and L2L 0.095 and 0.111 → 0.081 and 0.095). From p = 16 on one CTA
+// runs (of chunks of 16 two would fit at p = 16 by shared memory, and one by its 209 registers a thread). At p = 16 two
+// groups of warps with chunks of 24 share the rotations, one computing while the other scatters, as long as there
+// are pairs enough for that many chunks (6.04M pairs: 16.5 ms against 23.8 for one group; 1.05M: 3.83 against 4.31), one
 // group where there are not (71,365: 0.61 against 0.64; 56,448: 0.46 against 0.64).
 void m2l_rot(State& S) {
   const bool many = (int64_t)S.plan->npairs * S.plan->cache->nexp >= 1000000;
   for_order(S.plan->cache->p, [&](auto order) {
     constexpr int P = decltype(order)::value;
-    if constexpr (P <= 11) launch<P, 3, 1, 4, 4>(S);
-    else if constexpr (P <= 15) launch<P, 3, 1, 6, 2>(S);
+    if constexpr (P <= 11) launch<P, 3, 1, 4, rot_resident(P, 3, 1, 4)>(S);
+    else if constexpr (P <= 15) launch<P, 3, 1, 6, rot_resident(P, 3, 1, 2)>(S);
     else if (P == 16 && many) launch<16, 3, 2, 6, 1>(S);
     else launch<P, 2, 1, 8, 1>(S);
   });

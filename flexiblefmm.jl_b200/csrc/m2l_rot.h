@@ -30,6 +30,33 @@ struct RotLayout {
   }
 };
 
+// The tile's row of one pair: degree l from base(l) on, the l + 1 real parts of m = 0..l, then the l
+// imaginary parts; base(l) ≡ l (mod 4) and a row is an odd multiple of 4 doubles, so that the 8 pairs ×
+// 4 orders (or 4 degrees of one order) a warp reads or writes at once lie in distinct banks
+__host__ __device__ constexpr int rot_base(int l) { return l * l + 2 * (l / 2); }
+__host__ __device__ constexpr int rot_row(int p) { return (rot_base(p + 1) + 3) / 4 * 4 | 4; }
+// the row of the pair's (cos mφ, sin mφ): zeros past m = p for the padded inputs
+__host__ __device__ constexpr int rot_cs(int p) { return (p + 4) / 8 * 8 + 5; }
+constexpr int rot_list(int nc) { return 4 * nc + 2; }   // source, offset (bit 31: it points down), target, runs; the last run's end, their count
+
+// fragments of a class's translations; its rotations have twice as many (RotLayout's nt and nd)
+constexpr int rot_fragments(int p) {
+  int n = 0;
+  for (int s = 1; s <= p + 1; ++s) n += RotLayout::ksteps(s) * RotLayout::tiles(s);
+  return n;
+}
+// the shared memory of a CTA: G groups of warps, NG groups of 8 pairs a chunk each
+constexpr size_t rot_smem(int p, int NG, int G) {
+  const int nc = 8 * NG, nt = rot_fragments(p);
+  return sizeof(double) * ((size_t)32 * (2 * nt + G * nt) + (size_t)G * nc * (2 * rot_cs(p) + rot_row(p)) + 8) +
+         sizeof(int) * (size_t)G * 2 * rot_list(nc);
+}
+// the CTAs of an SM: `most` (what the registers allow), or as many as fit its 228 KB, 1 KB of each the system's
+constexpr int rot_resident(int p, int NG, int G, int most) {
+  const int fit = (int)(size_t(228 * 1024) / (rot_smem(p, NG, G) + 1024));
+  return fit < most ? fit : most;
+}
+
 struct RotHost {
   RotLayout layout;
   // per class of the far offsets, and (the last) for the direction (1, 1, 1) of the child slots:

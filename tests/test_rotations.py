@@ -1,6 +1,6 @@
 """The host tables of the FP64 translations by rotations (rotations.cpp), compiled here with g++: the
 blocks against projections of the rotated harmonics onto the harmonics by quadrature, in extended
-precision, and the time that the first state of an order waits for them.
+precision, the time that the first state of an order waits for them, and the CTAs of the translations that an SM holds.
 
 Bar: the tables are rounded once from extended precision, entries are at most 2 in magnitude (half an ulp
 is 2⁻⁵³ below 2), and the quadrature's own error stays below 1e-17, so 1.2e-16.
@@ -21,6 +21,7 @@ MAIN = r"""
 using namespace fmmb;
 int main(int, char** v) {
   const int p = atoi(v[1]);
+  printf("fit %d %zu\n", rot_resident(p, 3, 1, 99), rot_smem(p, 3, 1));
   const HostOperators op = build_operators(p, 1.0);
   const auto t0 = std::chrono::steady_clock::now();
   const auto h = rotation_tables(p, op);
@@ -48,12 +49,13 @@ def tables(tmp_path_factory):
 
     def run(p):
         out = subprocess.run([str(d / "main"), str(p)], check=True, capture_output=True, text=True).stdout
+        fit, out = out.split("\n", 1)
         ms, *parts = re.split(r"^class ", out, flags=re.M)
         classes = []
         for part in parts:
             head, *vals = part.strip().split("\n")
             classes.append((tuple(map(int, head.split())), np.array(vals, np.float64)))
-        return float(ms.split()[1]), classes
+        return float(ms.split()[1]), classes, tuple(map(int, fit.split()[1:]))
 
     return run
 
@@ -87,7 +89,7 @@ def legendre(n):
 
 @pytest.mark.parametrize("p", [1, 2, 5, 9])
 def test_blocks_are_the_projections(tables, p):
-    _, classes = tables(p)
+    _, classes, _ = tables(p)
     assert len(classes) == 35
     t, wt = legendre(p + 1)
     nph = 2 * p + 2
@@ -117,3 +119,11 @@ def test_first_state_does_not_wait_for_the_tables(tables):
     """They cost less than the dense operators that a cache builds anyway: 5 ms at the largest order (84 ms the
     operators), 292 by quadrature; the bar leaves room for a loaded machine."""
     assert min(tables(20)[0] for _ in range(3)) < 60
+
+
+def test_ctas_that_fit_an_sm(tables):
+    """The launches count on four CTAs an SM up to p = 10 and on three at p = 11 (chunks of 24 pairs)."""
+    fits = {p: tables(p)[2] for p in (1, 10, 11, 12, 15)}
+    for p, (fit, smem) in fits.items():
+        assert fit * (smem + 1024) <= 228 * 1024 < (fit + 1) * (smem + 1024)
+    assert fits[1][0] >= 4 and fits[10][0] == 4 and fits[11][0] == 3 and fits[12][0] == fits[15][0] == 2
