@@ -135,6 +135,7 @@ void build_blocks(Plan& P, int TB) {
   P.h_blocks.clear();
   P.level_pairs.assign(L, 0);
   int64_t base = 0;
+  P.max_block_pairs = 0;
   require(L < 256, FMMB_ERR_ARGUMENT, "too many levels");
   for (int q = 0; q < P.nseg; ++q) {
     const int l = P.seg_level[q], end = P.seg_start[q + 1];
@@ -147,6 +148,7 @@ void build_blocks(Plan& P, int TB) {
       P.h_blocks.push_back({l, q, b0, c, (int)base});
       base += np;
       P.level_pairs[l] += np;
+      P.max_block_pairs = std::max(P.max_block_pairs, np);
     }
   }
   require(base < (1ll << 31), FMMB_ERR_ARGUMENT, "too many far pairs for 32-bit offsets");

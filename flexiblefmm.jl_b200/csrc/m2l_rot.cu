@@ -534,18 +534,26 @@ RotSched schedule(const RotLayout& lay, int nw) {
   return s;
 }
 
-// The parts a block is cut into: more of them fill the device (`slots` groups run at once), fewer
-// of them fill the chunks (a class's last chunk of a part is half empty on average, and one with
-// few pairs costs a whole one): the power of two with the least waves × chunks per part. Measured with
-// the products on the FMA units at 6.04M far pairs of 293 blocks, p = 10 (1, 2, 4, 8 parts): 7.9, 6.0,
-// 6.0, 6.3 ms; at 207,331 pairs of a sphere: 0.77, 0.59, 0.72, 0.95 ms.
-int parts_per_block(const Plan& P, int nexp, int slots, int nc) {
+// The parts a block is cut into: more of them fill the device and cut the heaviest block (a cluster's hold twenty
+// times the average), fewer of them fill the chunks (a class's last chunk of a part is half empty, and one with
+// few pairs costs a whole one): the power of two with the least time, in chunks per class, of all parts over the
+// groups of warps that run at once (`slots`, `per_sm` of them on an SM) and of the heaviest block's on its own (the
+// fewer groups share its SM, the faster it runs: a twelfth per group). Of a class's λ pairs on average, a part has
+// any with probability 1 − e^−λ. Fitted to every power of two at 315 sets (p = 4 to 20; 1,200 to 400,000 points,
+// uniform, on a sphere and in clusters; ppl 24 to 300): 2 % above the best of them on average, and nowhere above the
+// rule that looked at the average block alone, which took up to 2.8 times the best. M2L, that rule → this: 150,000 points
+// in clusters p = 8 3.29 → 1.93 ms, p = 14 4.99 → 3.43, p = 20 15.9 → 8.1; uniform clouds and spheres within 1 %.
+int parts_per_block(const Plan& P, int nexp, int slots, int per_sm, int nc) {
   const double nb = (double)P.h_blocks.size();
   int best = 1;
   double least = 1e300;
   for (int sub = 1; sub <= P.TB / 4; sub *= 2) {
-    const double pairs = (double)P.npairs / (nb * sub * NCLASS);
-    const double t = std::max(1.0, nb * sub * nexp / slots) * std::max(1.0, pairs / nc + 0.5);
+    auto chunks = [&](double pairs, double last) {
+      const double lam = pairs / (sub * NCLASS), any = 1 - std::exp(-lam);
+      return std::max(any, lam / nc + last * any);
+    };
+    const double t = std::max(nb * sub * nexp / slots * chunks(P.npairs / nb, 0.75),
+                              chunks((double)P.max_block_pairs, 0.5) / (1 + 0.08 * (per_sm - 1)));
     if (t < 0.97 * least) { least = t; best = sub; }
   }
   return best;
@@ -581,7 +589,7 @@ void launch(State& S) {
   const int nb = (int)P.h_blocks.size();
   if (nb == 0) return;
   RotArgs A = common_args(S, K.rot_csf.p, S.M.p, S.Pl.p);
-  A.sub = parts_per_block(P, K.nexp, P.ctx->num_sms * MINB * G, 8 * NG);
+  A.sub = parts_per_block(P, K.nexp, P.ctx->num_sms * MINB * G, MINB * G, 8 * NG);
   A.nparts = nb * A.sub;
   A.TB = P.TB;
   A.blocks = P.blocks.p;
@@ -698,10 +706,11 @@ void l2l_rot(State& S, int l) { sweep<ROT_L2L>(S, l, S.plan->lv_rot_l2l[l - 1]);
 // with the registers and parts of four; M2M and L2L 0.095 and 0.111 → 0.081 and 0.095). From p = 16 on one CTA
 // runs (of chunks of 16 two would fit at p = 16 by shared memory, and one by its 209 registers a thread). At p = 16 two
 // groups of warps with chunks of 24 share the rotations, one computing while the other scatters, as long as there
-// are pairs enough for that many chunks (6.04M pairs: 16.5 ms against 23.8 for one group; 1.05M: 3.83 against 4.31), one
-// group where there are not (71,365: 0.61 against 0.64; 56,448: 0.46 against 0.64).
+// are pairs enough for that many chunks (one group's time over two groups': uniform clouds 0.55 at 56,448 pairs, 0.84 at
+// 184,722, 1.03 at 601,701, 1.09 at 640,584, 1.37 at 2.3M; spheres 0.94 at 308,559, 1.07 at 668,268, 1.19 at 1.4M; Gaussian
+// mixtures 0.94 at 381,317, 0.96 at 627,320, 1.05 at 1.06M, 1.34 at 3.1M).
 void m2l_rot(State& S) {
-  const bool many = (int64_t)S.plan->npairs * S.plan->cache->nexp >= 1000000;
+  const bool many = (int64_t)S.plan->npairs * S.plan->cache->nexp >= 600000;
   for_order(S.plan->cache->p, [&](auto order) {
     constexpr int P = decltype(order)::value;
     if constexpr (P <= 11) launch<P, 3, 1, 4, rot_resident(P, 3, 1, 4)>(S);

@@ -129,7 +129,7 @@ struct Plan {
   DBuf<int2> pairs;
   DBuf<int> rtab;                         // nblocks × 34 × TB: per class and target, count << 16 | offset in the class
   DBuf<int> rounds;                       // nblocks × 34: per class the largest count of a target
-  int64_t npairs = 0;
+  int64_t npairs = 0, max_block_pairs = 0;
   std::vector<int64_t> level_pairs;       // far pairs per level
   std::vector<int> h_pair_count;          // far pairs per target node (the blocks are cut from it)
   DBuf<double> d_scale, d_m2l_scale;      // per level

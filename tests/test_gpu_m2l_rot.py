@@ -30,7 +30,7 @@ def test_rotated_m2l_matches_dense(oracle, fmmb, p):
 
 
 def test_order_16_same_in_a_large_launch(fmmb):
-    """At p = 16 a launch of a million pairs or more takes another shape (two groups of warps, chunks of
+    """At p = 16 a launch of 600,000 pairs or more takes another shape (two groups of warps, chunks of
     24 pairs). A pair's product and the order of a target's sums depend on neither: a batch of eight
     instances, large, equals each instance's own plan, small, bit by bit."""
     rng = np.random.default_rng(16)
@@ -40,8 +40,25 @@ def test_order_16_same_in_a_large_launch(fmmb):
     batch = fmmb.BatchFMM(m, sets, ppl=4, bbox=BOX)
     cache = fmmb.OperatorCache(m)
     alone = [fmmb.FMM(m, s, ppl=4, bbox=BOX, cache=cache) for s in sets]
-    assert max(f.npairs for f in alone) < 1000000 <= batch.npairs
+    assert max(f.npairs for f in alone) < 600000 <= batch.npairs
     u, g = fmmb.evaluate_at_sources_both(batch, fmmb.build_expansions(batch, batch.sources, batch.concat(tau)))
     for i, f in enumerate(alone):
         a, b = fmmb.evaluate_at_sources_both(f, fmmb.build_expansions(f, sets[i], tau[i]))
+        assert np.array_equal(batch.split(u)[i], a) and np.array_equal(batch.split(g)[i], b)
+
+
+@pytest.mark.parametrize("p", [4, 8, 11, 14, 20])
+def test_same_bits_whatever_the_parts(fmmb, p):
+    """A skewed tree's blocks are cut into more parts than a uniform one's (the heaviest block decides): an instance
+    of a batch whose other instance is one dense cluster equals its own plan bit by bit."""
+    rng = np.random.default_rng(50 + p)
+    m = fmmb.SphericalHarmonics(fmmb.Laplace3D(), p=p)
+    sets = [rng.random((3000, 3)), np.clip(0.5 + 0.02 * rng.standard_normal((20000, 3)), 0.0, 1.0)]
+    tau = [rng.standard_normal(len(s)) for s in sets]
+    batch = fmmb.BatchFMM(m, sets, ppl=16, bbox=BOX)
+    cache = fmmb.OperatorCache(m)
+    u, g = fmmb.evaluate_at_sources_both(batch, fmmb.build_expansions(batch, batch.sources, batch.concat(tau)))
+    for i, s in enumerate(sets):
+        f = fmmb.FMM(m, s, ppl=16, bbox=BOX, cache=cache)
+        a, b = fmmb.evaluate_at_sources_both(f, fmmb.build_expansions(f, s, tau[i]))
         assert np.array_equal(batch.split(u)[i], a) and np.array_equal(batch.split(g)[i], b)
