@@ -15,6 +15,7 @@
 //   L2T (a22)   the surface sums of the leaves' local densities (eval.cu) and the near field
 // The operators are built at width 1 (Laplace3D is homogeneous of degree −1): at width w the
 // surfaces scale by w, the pseudo-inverses by w and the M2L tables by 1/w.
+#include <algorithm>
 #include <map>
 #include <tuple>
 
@@ -110,10 +111,11 @@ __global__ void __launch_bounds__(128) k_ki_check(const int* __restrict__ nodes,
 __global__ void __launch_bounds__(128) k_ki_forward(int first, int p, int ns, int LD, int nfp,
                                                     const uint8_t* __restrict__ flags, const double* __restrict__ M,
                                                     const float2* __restrict__ tw, const int* __restrict__ embed,
-                                                    float2* __restrict__ spec) {
+                                                    float2* __restrict__ spec, int* __restrict__ next) {
   extern __shared__ float2 smf[];
   __shared__ float2 c_tw[SIDE * SIDE];              // [j·n + k] = e^{−2πi jk/n}, n = 2p
   const int g = first + blockIdx.x, n = 2 * p, nh = p + 1, tid = threadIdx.x;
+  if (blockIdx.x == 0 && tid < nfp / FB) next[tid] = 0;   // the Hadamard sums' hand-out, before them on the stream
   if (!(flags[g] & F_SOURCE)) return;
   float2* a1 = smf;                                 // [nh·p·p]
   float2* a2 = a1 + nh * p * p;                     // [nh·n·p]
@@ -183,20 +185,23 @@ __device__ __forceinline__ void ki_fma2(uint64_t& d, uint64_t a, uint64_t b) {
   asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
 }
 
-// Hadamard sums: CTA (frequency block fb, range of sibling groups); the 316 tables' block fb in shared
-// memory; a warp per group, lane l the frequencies 2l, 2l + 1 of the block. The eight siblings' far
+// Hadamard sums: a CTA keeps the 316 tables' block fb = blockIdx.x in shared memory, one CTA an SM; a warp per
+// sibling group, lane l the frequencies 2l, 2l + 1 of the block. The eight siblings' far
 // sources are the sourced children of their parent's colleagues, so each source's spectrum is read once
 // and multiplied into every sibling it is far from (seven of eight on average, in registers): what
 // bounds the sums is the L1 / shared-memory pipe, and a pair moves one table entry and an eighth of a
 // spectrum through it in place of one of each, with half the multiply-add instructions (f32x2).
-// The groups of a CTA are handed out one by one, and a colleague's spectra are loaded during the sums of the
-// one before. Measured, the M2L stage at 300,000 clustered points (3.63M pairs): p = 4 a warp per target 1.73
-// ms, sibling groups and no transforms of empty nodes 1.48, with the hand-out and the loads ahead 1.36; p = 8 the
-// last two 7.87 and 6.45.
+// Each block's groups are handed out one by one to the warps of all its CTAs (next[fb]: they differ by a factor of
+// ten in far sources), and a colleague's spectra are loaded during the sums of the one before. Measured, the M2L
+// stage at 300,000 clustered points (3.63M pairs): p = 4 a warp per target 1.73 ms, sibling groups and no transforms
+// of empty nodes 1.48, with the hand-out and the loads ahead 1.36; p = 8 the last two 7.87 and 6.45. With the groups in fixed
+// shares of 128 to a CTA, ghosts among them, small and uniform trees left most SMs idle and were slower than a warp per
+// target (a warp per target, fixed shares, this: 60,000 uniform points p = 4 0.278, 0.640, 0.190; 20,000 p = 8 0.204,
+// 0.296, 0.159; 60,000 clustered p = 2 0.560, 0.867, 0.284; 500,000 clustered p = 8 17.4, 11.5, 10.7).
 // fidx: per colleague offset (27), source child and target child the far offset's index, −1 when near.
-__global__ void __launch_bounds__(HAD_THREADS) k_ki_hadamard(int ngroups, int per_cta, int nfp,
+__global__ void __launch_bounds__(HAD_THREADS) k_ki_hadamard(int ngroups, int* __restrict__ next, int nfp,
                                                              const int2* __restrict__ groups,
-                                                             const int* __restrict__ ptr, const int4* __restrict__ cell,
+                                                             const int4* __restrict__ cell,
                                                              const int* __restrict__ cf, const int* __restrict__ col,
                                                              const uint8_t* __restrict__ flags,
                                                              const int16_t* __restrict__ fidx,
@@ -204,24 +209,24 @@ __global__ void __launch_bounds__(HAD_THREADS) k_ki_hadamard(int ngroups, int pe
                                                              const float2* __restrict__ spec, float2* __restrict__ U) {
   extern __shared__ float4 st[];   // [NFAR][FB / 2]: (re, re, im, im) of a frequency pair
   int16_t* sf = reinterpret_cast<int16_t*>(st + NFAR * (FB / 2));   // [27][8][8]
-  __shared__ int next;
   const int fb = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
+  __shared__ int done;                               // a CTA that starts when the others are done
+  if (tid == 0) done = *(volatile int*)(next + fb) >= ngroups;
+  __syncthreads();
+  if (done) return;
   for (int i = tid; i < NFAR * (FB / 2); i += HAD_THREADS) {
     const int f = i / (FB / 2), l = i % (FB / 2);
     const float4 v = reinterpret_cast<const float4*>(tab + (int64_t)f * nfp + fb * FB)[l];
     st[i] = make_float4(v.x, v.z, v.y, v.w);
   }
   for (int i = tid; i < NCOL * NCH * NCH; i += HAD_THREADS) sf[i] = fidx[i];
-  if (tid == 0) next = 0;
   __syncthreads();
-  const int q0 = blockIdx.y * per_cta, q1 = min(ngroups, q0 + per_cta);
-  for (;;) {                                         // the CTA's groups handed out one by one: they differ by a factor of ten
+  for (;;) {
     int q = 0;
-    if (lane == 0) q = q0 + atomicAdd(&next, 1);
+    if (lane == 0) q = atomicAdd(next + fb, 1);
     q = __shfl_sync(0xffffffffu, q, 0);
-    if (q >= q1) break;
+    if (q >= ngroups) break;
     const int2 gr = groups[q];                       // parent, first sibling
-    if (ptr[gr.y] == ptr[gr.y + NCH]) continue;      // no far pairs
     // lane k: colleague k of the parent, its children and which of them have sources
     int s0 = -1, o = 0, mask = 0;
     if (lane < NCOL) {
@@ -413,11 +418,12 @@ void ki_prepare(Plan& P) {
   P.lv_m2m.assign(P.L, C.ki_m2m.p);
   P.lv_l2l.assign(P.L, C.ki_l2l.p);
   build_target_pairs(P);
-  std::vector<int2> groups;                 // the sibling groups of the levels with far pairs
+  std::vector<int2> groups;                 // the sibling groups with far pairs (half of an adaptive tree's are ghosts)
   for (int l = 2; l < P.L; ++l)
     for (int g = 0; g < P.level_groups[l]; ++g) {
       const int c0 = P.level_start[l] + NCH * g;
-      groups.push_back(make_int2(P.h_parent[c0], c0));
+      if (std::any_of(&P.h_pair_count[c0], &P.h_pair_count[c0] + NCH, [](int n) { return n > 0; }))
+        groups.push_back(make_int2(P.h_parent[c0], c0));
     }
   P.n_ki_groups = (int)groups.size();
   to_device(P.ki_groups, groups, s);
@@ -439,6 +445,7 @@ void ki_state(State& S) {
   S.ki_ll.alloc((size_t)P.nnodes * C.ki_nld);
   S.ki_spec.alloc((size_t)P.nnodes * C.ki_nfp);
   S.ki_u.alloc((size_t)P.nnodes * C.ki_nfp);
+  S.ki_next.alloc(C.ki_nfp / FB);
 }
 
 // P2M: check potentials, then the multipoles V·(S⁺Uᴴ·check) of the childless nodes
@@ -470,15 +477,16 @@ int ki_m2l(State& S) {
   const size_t fsm = sizeof(float2) * (nh * p * p + nh * n * p) + sizeof(float) * p * p * p;
   FMMB_CUDA(cudaFuncSetAttribute(k_ki_forward, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm));
   k_ki_forward<<<nt, 128, fsm, s>>>(first, p, C.np, C.ld, C.ki_nfp, P.flags.p, S.M.p, C.ki_tw.p, C.ki_embed.p,
-                                     S.ki_spec.p);
+                                     S.ki_spec.p, S.ki_next.p);
   FMMB_LAUNCH_CHECK();
   const size_t hsm = sizeof(float4) * NFAR * (FB / 2) + sizeof(int16_t) * NCOL * NCH * NCH;
   FMMB_CUDA(cudaFuncSetAttribute(k_ki_hadamard, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)hsm));
   if (P.n_ki_groups > 0) {
-    const int per_cta = 128;
-    k_ki_hadamard<<<dim3(C.ki_nfp / FB, (P.n_ki_groups + per_cta - 1) / per_cta), HAD_THREADS, hsm, s>>>(
-        P.n_ki_groups, per_cta, C.ki_nfp, P.ki_groups.p, P.tp_ptr.p, P.cell.p, P.cf.p, P.col.p, P.flags.p, C.ki_fidx.p,
-        C.ki_tab.p, S.ki_spec.p, S.ki_u.p);
+    // CTAs for two waves: the second's join the blocks that are not done, or leave at once
+    const int blocks = C.ki_nfp / FB, ctas = std::min(P.n_ki_groups, (2 * P.ctx->num_sms + blocks - 1) / blocks);
+    k_ki_hadamard<<<dim3(blocks, ctas), HAD_THREADS, hsm, s>>>(
+        P.n_ki_groups, S.ki_next.p, C.ki_nfp, P.ki_groups.p, P.cell.p, P.cf.p, P.col.p, P.flags.p, C.ki_fidx.p, C.ki_tab.p,
+        S.ki_spec.p, S.ki_u.p);
     FMMB_LAUNCH_CHECK();
   }
   const size_t ism = sizeof(float2) * (nh * n * n + nh * n * p + nh * p * p) + sizeof(float) * p * p * p;

@@ -200,6 +200,7 @@ struct State {
   // surfaces (nnodes × NLD), the spectra of the multipoles and of the M2L sums (nnodes × nfp)
   DBuf<double> ki_pm, ki_y, ki_ll;
   DBuf<float2> ki_spec, ki_u;
+  DBuf<int> ki_next;                      // per frequency block of the Hadamard sums the groups handed out
   bool built = false;
   // the side stream of the split matvec (the near field beside the passes) and its two events,
   // created on first use

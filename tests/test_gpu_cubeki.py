@@ -135,3 +135,34 @@ def test_ki_matches_oracle(oracle, fmmb, p, precision):
         assert np.array_equal(t[k], getattr(T, k)), k
     bar = 2e-6 if precision == "fp64" else 2e-5
     assert np.linalg.norm(u - ou) / np.linalg.norm(ou) < bar
+
+
+@pytest.mark.parametrize("p,n,gen", [(2, 700, uniform3), (3, 4000, uniform3), (4, 40000, uniform3), (4, 20000, clustered3)])
+def test_ki_hadamard_hand_out(fmmb, p, n, gen):
+    """The sibling groups handed out over the CTAs of a frequency block, from fewer groups than warps up to several
+    per warp: the counters start anew on every build (the same bits again), each target with far pairs gets its
+    sum, no other does."""
+    rng = np.random.default_rng(40 + p)
+    pts, tau = gen(rng, n), rng.standard_normal(n)
+    m = fmmb.CubeKernelIndependent(fmmb.Laplace3D(), p=p)
+    f = fmmb.FMM(m, pts, ppl=30, bbox=((0.0, 0.0, 0.0), 1.0))
+    st = fmmb.build_expansions(f, pts, tau)
+    u = fmmb.evaluate_at_sources(f, st)
+    M, Lc = st.expansions()
+    for _ in range(3):
+        fmmb.build_expansions_(st, f, pts, tau)
+        assert np.array_equal(fmmb.evaluate_at_sources(f, st), u)
+    fmmb.build_expansions_(st, f, pts, -2.0 * tau)             # exact in every format: no sum is left from before
+    assert np.array_equal(fmmb.evaluate_at_sources(f, st), -2.0 * u)
+    t = f.tree()
+    with_pairs = np.zeros(f.nnodes, bool)
+    with_pairs[np.concatenate([f.pairs(l)[0] for l in range(2, f.nlevels)])] = True
+    leaf = t["leaf"].astype(bool)                              # expansions() gives the leaves' local expansions
+    assert np.all(np.any(Lc[with_pairs & leaf] != 0, axis=1))
+    if f.nlevels == 3:
+        assert not np.any(Lc[~with_pairs])
+    sel = np.sort(rng.choice(n, 200, replace=False))
+    r = np.linalg.norm(pts[sel][:, None, :] - pts[None, :, :], axis=2)
+    r[np.arange(200), sel] = np.inf
+    # the method's error falls about five-fold per point of the edge (p = 8: 1e-6): 3e-2 at p = 2
+    assert rel_l2(u[sel], KC * (tau[None, :] / r).sum(1)) < 0.15 / 5 ** (p - 1)
