@@ -210,17 +210,11 @@ void finish_plan(fmmb_cache* cache, std::unique_ptr<fmmb_plan>& h, const double*
   }
   // the translation operators of every level: the cache's (homogeneous kernels), or the
   // level width's own (Yukawa3D, built on first use)
-  P.lv_reps.assign(P.L, C.reps.p);
   P.lv_m2m.assign(P.L, C.m2m.p);
   P.lv_l2l.assign(P.L, C.l2l.p);
   if (C.kernel == FMMB_KERNEL_YUKAWA3D) yukawa_prepare(P);
-  {
-    std::vector<uint64_t> t(P.L);
-    for (int l = 0; l < P.L; ++l) t[l] = (uint64_t)(uintptr_t)P.lv_reps[l];
-    to_device(P.d_lv_reps, t, ctx.stream);
-  }
   build_lists(P);
-  if (C.method == FMMB_METHOD_CUBE_KI) ki_prepare(P);   // its operators, its target-major pairs
+  if (C.method == FMMB_METHOD_CUBE_KI) ki_prepare(P);   // its operators, its sibling groups
   if (C.method == FMMB_METHOD_KI_CIRCLE) kic_prepare(P);
   h->parent = cache;
   std::lock_guard<std::mutex> lk(g_handles);

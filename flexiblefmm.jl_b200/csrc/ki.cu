@@ -417,7 +417,7 @@ void ki_prepare(Plan& P) {
   }
   P.lv_m2m.assign(P.L, C.ki_m2m.p);
   P.lv_l2l.assign(P.L, C.ki_l2l.p);
-  build_target_pairs(P);
+  build_target_pairs(P, false);
   std::vector<int2> groups;                 // the sibling groups with far pairs (half of an adaptive tree's are ghosts)
   for (int l = 2; l < P.L; ++l)
     for (int g = 0; g < P.level_groups[l]; ++g) {

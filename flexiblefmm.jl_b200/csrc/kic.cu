@@ -63,11 +63,8 @@ __global__ void __launch_bounds__(128) k_kic_check(const int* __restrict__ nodes
   }
 }
 
-// the dense M2L: warp per target t, Pl[t] = Σ over its far pairs (s, f) of A_f(level) · M[s]
-// (rows lane and lane + 32; the columns of M[s] broadcast by shuffles). Only the in-plane offsets have a
-// map: the far offsets are listed by layers of oz, and those of oz = 0 are the 40 after 98 + 40 others. The
-// pairs of the embedding's off-plane boxes, half of all pairs or more, are passed over.
-constexpr int INPLANE0 = 138, INPLANE = 40;
+// the dense M2L: warp per target t, Pl[t] = Σ over its far pairs in the plane (s, f) of A_f(level) · M[s]
+// (rows lane and lane + 32; the columns of M[s] broadcast by shuffles)
 __global__ void __launch_bounds__(128) k_kic_m2l(int first, int last, int N, const int* __restrict__ ptr,
                                                  const int2* __restrict__ tp, const int4* __restrict__ cell,
                                                  const uint64_t* __restrict__ ops_lv, const double* __restrict__ M,
@@ -80,7 +77,6 @@ __global__ void __launch_bounds__(128) k_kic_m2l(int first, int last, int N, con
   double a0 = 0, a1 = 0;
   for (int k = k0; k < k1; ++k) {
     const int2 pr = tp[k];
-    if ((unsigned)(pr.y - INPLANE0) >= (unsigned)INPLANE) continue;
     const double* A = ops + (int64_t)pr.y * CLD * CLD;
     const double* x = M + (int64_t)pr.x * CLD;
     const double xl = x[lane], xh = x[lane + 32];
@@ -115,6 +111,7 @@ void kic_prepare(Plan& P) {
   P.kic_upsu.assign(P.L, nullptr);
   P.kic_downv.assign(P.L, nullptr);
   P.kic_downsu.assign(P.L, nullptr);
+  std::vector<uint64_t> t(P.L, 0);
   {
     std::lock_guard<std::mutex> lk(C.mu);
     for (int l = 2; l < P.L; ++l) {
@@ -134,7 +131,7 @@ void kic_prepare(Plan& P) {
         it = C.kic_levels.emplace(e, std::move(d)).first;
       }
       const Cache::CircleLevel& d = *it->second;
-      P.lv_reps[l] = d.m2l.p;
+      t[l] = (uint64_t)(uintptr_t)d.m2l.p;
       P.lv_m2m[l] = d.m2m.p;
       P.lv_l2l[l] = d.l2l.p;
       P.kic_upv[l] = d.upv.p;
@@ -143,10 +140,8 @@ void kic_prepare(Plan& P) {
       P.kic_downsu[l] = d.downsu.p;
     }
   }
-  std::vector<uint64_t> t(P.L);
-  for (int l = 0; l < P.L; ++l) t[l] = (uint64_t)(uintptr_t)P.lv_reps[l];
-  to_device(P.d_lv_reps, t, s);
-  build_target_pairs(P);
+  to_device(P.kic_m2l, t, s);
+  build_target_pairs(P, true);
   // the childless sourced nodes and every real leaf, with their level ranges
   std::vector<int> s2m, all;
   for (int g = 0; g < P.nnodes; ++g) {
@@ -198,7 +193,7 @@ int kic_m2l(State& S) {
   const int first = P.level_start[std::min(2, P.L)], last = P.nnodes;
   if (last <= first) return 0;
   k_kic_m2l<<<nblk(last - first, 4), 128, 0, P.ctx->stream>>>(first, last, C.np, P.tp_ptr.p, P.tp.p, P.cell.p,
-                                                              P.d_lv_reps.p, S.M.p, S.Pl.p);
+                                                              P.kic_m2l.p, S.M.p, S.Pl.p);
   FMMB_LAUNCH_CHECK();
   return 1;
 }

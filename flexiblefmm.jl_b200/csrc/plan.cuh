@@ -133,11 +133,9 @@ struct Plan {
   std::vector<int64_t> level_pairs;       // far pairs per level
   std::vector<int> h_pair_count;          // far pairs per target node (the blocks are cut from it)
   DBuf<double> d_scale, d_m2l_scale;      // per level
-  // the translation operators of each level (the cache's for the homogeneous kernels; the
-  // level's own width for Yukawa3D): M2L representatives, M2M into and L2L out of the level's
-  // nodes; the representatives' table on the device for the M2L kernel; Yukawa3D's κ̂² per level
-  std::vector<const double*> lv_reps, lv_m2m, lv_l2l;
-  DBuf<uint64_t> d_lv_reps;
+  // the dense translation operators of each level (the cache's for the homogeneous kernels; the
+  // level's own width for Yukawa3D): M2M into and L2L out of the level's nodes; Yukawa3D's κ̂² per level
+  std::vector<const double*> lv_m2m, lv_l2l;
   DBuf<double> d_kh2;
   // per level the translations along z: of the classes (a table on the device), into the level's
   // nodes from their children, out of the level's nodes into theirs
@@ -148,7 +146,8 @@ struct Plan {
   // state; the Yukawa levels they come from stay held by the plan
   DBuf<uint64_t> d_lv_reps16, d_lv_rsc;
   std::vector<std::shared_ptr<YukawaLevel>> lv_yukawa;
-  // the kernel-independent method: every target's far pairs (source, far index), target-major
+  // the kernel-independent methods: the first of each target's far pairs; on circles those in the plane (source,
+  // far index), target-major
   DBuf<int> tp_ptr;
   DBuf<int2> tp;
   DBuf<int> ki_leaves;                    // every real leaf (with sources or not)
@@ -158,6 +157,7 @@ struct Plan {
   // the circle method: per level its pseudo-inverse factors, and the level ranges of the
   // childless nodes with sources and of the real leaves (both lists are in node order)
   std::vector<const double*> kic_upv, kic_upsu, kic_downv, kic_downsu;
+  DBuf<uint64_t> kic_m2l;                 // and its M2L maps, a table on the device
   std::vector<int> s2m_level_start, ki_leaf_level_start;
   // per level its sibling groups: the level's first 8·level_groups[l] nodes (a batch's roots
   // below level 0 follow them)
@@ -235,7 +235,7 @@ int tuned_block_size(const Plan& P);
 // (tune_blocks: also the plan's M2L block size, shared by the plan's other states); out: the
 // chosen block size, 0, 4 (warps of a near-field team), and the M2L and near-field ms
 void autotune(State& S, const double* xyz_dev, const double* tau_dev, bool tune_blocks, double* out);
-void build_target_pairs(Plan& P);
+void build_target_pairs(Plan& P, bool plane);
 // passes.cu
 void upload_operators(Cache& C);
 void gather_inputs(State& S, const double* xyz_dev, const double* tau_dev);
