@@ -254,15 +254,22 @@ constexpr size_t STORE_BYTES = size_t(4) << 30;
 std::mutex g_store_mu;
 std::map<std::tuple<int, int, double, double>, std::shared_ptr<YukawaLevel>> g_store;
 std::vector<std::tuple<int, int, double, double>> g_store_order;   // insertion order
-size_t g_store_bytes = 0;
 
-size_t level_bytes(const YukawaLevel& lv) { return lv.reps.bytes() + lv.m2m.bytes() + lv.l2l.bytes(); }
+// all of a width's operators, those that its states built later too (the mixed path's, the translations along z)
+size_t level_bytes(YukawaLevel& lv) {
+  std::lock_guard<std::mutex> lk(lv.mu);
+  const RotTrans& r = lv.rot_t;
+  return lv.reps.bytes() + lv.m2m.bytes() + lv.l2l.bytes() + lv.reps16.bytes() + lv.row_scale.bytes() + r.m2l.bytes() +
+         r.m2m.bytes() + r.l2l.bytes();
+}
 
 void store_trim() {
-  for (size_t i = 0; i < g_store_order.size() && g_store_bytes > STORE_BYTES;) {
+  size_t held = 0;
+  for (auto& e : g_store) held += level_bytes(*e.second);
+  for (size_t i = 0; i < g_store_order.size() && held > STORE_BYTES;) {
     auto it = g_store.find(g_store_order[i]);
     if (it != g_store.end() && it->second.use_count() == 1) {
-      g_store_bytes -= level_bytes(*it->second);
+      held -= level_bytes(*it->second);
       g_store.erase(it);
       g_store_order.erase(g_store_order.begin() + i);
     } else {
@@ -291,7 +298,6 @@ std::shared_ptr<YukawaLevel> level_operators(Cache& C, int e, cudaStream_t s) {
   g_alloc_stream = keep;
   g_store[key] = lv;
   g_store_order.push_back(key);
-  g_store_bytes += level_bytes(*lv);
   store_trim();
   return lv;
 }
