@@ -771,7 +771,7 @@ void prepare_mixed_operators(Cache& C) {
 // class operators (copied to the host once per width and shared by the plans that use it)
 void prepare_mixed_levels(Plan& P) {
   Cache& C = *P.cache;
-  if (P.d_lv_reps16.n == (size_t)P.L) return;
+  if (P.d_lv_rsc.n == (size_t)P.L) return;        // the last of the tables
   cudaStream_t s = P.ctx->stream;
   std::vector<uint64_t> r16(P.L, 0), rs(P.L, 0);
   for (int l = 0; l < P.L; ++l) {
@@ -783,7 +783,7 @@ void prepare_mixed_levels(Plan& P) {
     if (l >= (int)P.lv_yukawa.size() || !P.lv_yukawa[l]) continue;   // no far pairs on this level
     YukawaLevel& Y = *P.lv_yukawa[l];
     std::lock_guard<std::mutex> lk(Y.mu);
-    if (!Y.reps16.p) {
+    if (!Y.row_scale.p) {
       HostOperators op;
       op.p = C.p; op.np = C.np; op.ld = C.ld;
       op.reps = to_host(Y.reps.p, (size_t)NCLASS * C.ld * C.ld, s);
