@@ -79,7 +79,6 @@ int64_t bytes_estimate(int64_t n, int p, int ppl, int precision, int kernel) {
   int64_t b = n * (nexp == 4 ? 448 : 256);               // points in and sorted, keys, perm, densities, outputs
   b += nodes * (2 * nexp * ld * 8 + 27 * 4 + 64);        // multipoles, partial locals, colleagues, node arrays
   b += nodes * 190 * 8;                                  // far pairs
-  if (nexp == 4) b += nodes / 8 * 4 * 8 * ld * 8;        // M2M / L2L staging of the largest level
   if (precision == FMMB_PRECISION_MIXED) b += nodes * kp * 8 + nodes * 4;   // FP16 copies, scales
   return b + (16 << 20);
 }

@@ -127,3 +127,21 @@ def test_server_yukawa_requests(fmmb):
             du[k] = yukawa_direct(pts[m], tau[m], pts[i:i + 1], 5.0)[0]
         err = rel_l2(u[sel], du)
         assert err < (1e-8 if tol < 1e-8 else 3 * tol), (len(pts), tol, info["p"], err)
+
+
+def test_server_stokes_estimate_holds_four_expansions(fmmb):
+    """The estimate that admits a request grows, per point, by at most four times a Laplace request's of the same
+    order and leaf size: four expansions on one tree, and no staging beside them."""
+    rng = np.random.default_rng(21)
+    srv = fmmb.Server(0, slots=1)
+    per_point = []
+    for stokes in (False, True):
+        b = []
+        for n in (2000, 6000):
+            x = rng.random((n, 3))
+            k = srv.submit_stokes(x, rng.standard_normal((n, 3)), p=16, ppl=16) if stokes else \
+                srv.submit(x, rng.standard_normal(n), p=16, precision="fp64", ppl=16)
+            b.append(srv.wait(k)[2]["bytes_estimate"])
+        per_point.append((b[1] - b[0]) / 4000)
+    srv.close()
+    assert per_point[0] < per_point[1] <= 4 * per_point[0]
