@@ -248,12 +248,16 @@ __global__ void k_p2m_dipoles(const int* __restrict__ nodes, int nn, int p, cons
   M[(int64_t)node * pitch + k] += s * v;
 }
 
-// nodes [i0, i0 + nn) of the list; 16 nodes per CTA (4 where none share a warp) where there are CTAs enough
+// nodes [i0, i0 + nn) of the list: several per warp where there are CTAs enough for that (four per warp fill the
+// device from about 128 nodes an SM on; two that share a warp, on average, from 24; one from four, or from 32 where
+// nodes are large and the CTA's four would be taken one after the other by all its warps)
 template <int P, bool YK, typename R, bool MANY>
 void launch(State& S, int i0, int nn, const P2MSets& sets) {
   Plan& P_ = *S.plan;
-  const int ny = MANY ? 1 : sets.n, fill = 32 * P_.ctx->num_sms;
-  const int npw = P2MShape<P, YK, R>::PACK && (int64_t)nn * ny >= 4 * fill ? 4 : ((int64_t)nn * ny >= fill ? 1 : 0);
+  const int ny = MANY ? 1 : sets.n;
+  const int64_t per_sm = (int64_t)nn * ny / P_.ctx->num_sms, avg = P_.N / P_.n_s2m;
+  const bool pack = P2MShape<P, YK, R>::PACK;
+  const int npw = pack && per_sm >= 128 ? 4 : (pack && avg <= 16 && per_sm >= 24 ? 2 : per_sm >= (avg <= 32 ? 4 : 32));
   const int npc = npw ? P2M_WARPS * npw : 1;
   auto kern = k_p2m<P, YK, R, MANY>;
   constexpr size_t smem = P2MShape<P, YK, R>::smem(MANY);
