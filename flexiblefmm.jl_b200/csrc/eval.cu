@@ -1,8 +1,8 @@
 // Evaluation at the targets of one leaf (src/evaluate.jl:12-48, src/device.jl:89-100,185-206),
 // in two kernels:
-//   k_l2p   the far field: L2P of the leaf's local expansion (harmonics.jl:447-486), one warp
-//           per leaf group with the local staged in shared memory, lanes over the targets; FP64 on
-//           the plain path, FP32 on the mixed path (tolerances ≥ 1e-8); writes the outputs
+//   k_l2p   the far field: L2P of the leaf's local expansion (harmonics.jl:447-486), one warp per leaf group (a
+//           CTA of four where leaves are few) with the local staged in shared memory, lanes over the targets;
+//           FP64 on the plain path, FP32 on the mixed path (tolerances ≥ 1e-8); writes the outputs
 //   k_near  the near field (near.cuh): the sources of the 27 colleagues, flattened into batches of 32
 //           that the warps of a leaf's team stage in shared memory, lanes over the targets; adds to
 //           the outputs. The self term is skipped by index (evaluate_at_sources,

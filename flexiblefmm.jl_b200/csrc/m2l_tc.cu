@@ -24,8 +24,9 @@
 //     K-major canonical layout) into a ring: 8 lanes write the 8 rows of one 128-byte core
 //     matrix; odd quarter-turn rotations read a second copy of the multipoles in which the two
 //     entries of every odd-order pair are swapped, and the source-side signs cost one XOR on the way
-//     from the load's registers to shared memory. The gather's latency bounds the kernel (per round of
-//     128 pairs about 7,500 cycles at p = 11, of which the MMAs take 2,000), so its first loads are
+//     from the load's registers to shared memory. What bounds the kernel is the L1 / shared-memory pipe (75 %
+//     busy), most of it the gather's loads, stores and sign lookups, with their latency between the hand-offs (a
+//     round of 128 pairs takes about 7,500 cycles at p = 11, its MMAs 2,000): the first loads are
 //     issued before the slab's buffer is free, and where the ring holds fewer slabs than there are
 //     gather warps two warps share a slab. Measured (one warp a slab, cp.async into the slab and the
 //     signs in place → two warps → loads through registers): a million points p = 11 1.79 → 1.71 →
@@ -35,7 +36,7 @@
 //     copy (cp.async.bulk, no tensor map, no multicast) when the class changes, after the
 //     previous class's MMAs completed; then per K-step issues three MMAs (M = 128, N, K = 16)
 //     into one of two accumulator stages in tensor memory;
-//   - read-back warps (thread = target; two warps per TMEM lane quadrant, each half of the
+//   - read-back warps (thread = target; four warps per TMEM lane quadrant, each a quarter of the
 //     columns) apply the target-side permutation of the pair's element (odd-m entries take their
 //     partner's value for odd rotations, signs by XOR) and the source scale, and add the row into
 //     the target's class sums, kept in tensor memory; at the class's last round they add the sums,

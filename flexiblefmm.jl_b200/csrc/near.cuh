@@ -10,11 +10,12 @@
 // as much.) The warps' sums meet in shared memory in warp order. A leaf of at most NEAR_ALONE
 // source-target pairs goes to one warp: a team's set-up and sums would cost more than its share.
 // How the sums are split depends on the leaf's own targets and sources only, so a leaf's results are
-// the same in every plan that holds it. Groups per CTA (4 or 1) only place the work: 4 share the
+// the same in every plan that holds it; the last bits of a target's sum depend on how many targets share its leaf. Groups per CTA (4 or 1) only place the work: 4 share the
 // set-up's latency, 1 spreads few leaves over more SMs.
-// Bound by FP64 (FP32) issue where leaves are full. Measured, near field and L2P, a warp a leaf and no lane
-// splits → this: a million points FP64 ppl = 64 1.99 → 1.67 ms, in FP32 0.79 → 0.74; 400,000 points FP64
-// 0.60 → 0.49; a sphere of 31,000 FP64 ppl = 128 (few full leaves) 0.66 → 0.21; 300,000 points of a Gaussian
+// The arithmetic pipe and the issue slots are each about 60 % busy (a million points), the rest is the latency of a
+// pair's chain and the team's barriers. Measured, near field and L2P, a warp a leaf and no lane
+// splits → this: a million points FP64 ppl = 64 p = 10 2.16 → 1.79 ms, in FP32 p = 4 0.79 → 0.74; 200,000 points FP64
+// p = 4 0.70 → 0.45; a sphere of 30,000 FP64 ppl = 128 p = 16 (few full leaves) 0.68 → 0.21; 300,000 points of a Gaussian
 // mixture in FP32 (many small leaves) 0.335 → 0.318. NEAR_ALONE: with teams from 256 sources on instead, the
 // 400,000 FP64 points took 0.92, with every leaf alone the sphere's few leaves would leave SMs idle.
 //

@@ -310,7 +310,6 @@ __global__ void k_bounds_batch(const double* __restrict__ xyz, const int64_t* __
   if (threadIdx.x < 6) out[((int64_t)blockIdx.y * gridDim.x + blockIdx.x) * 6 + threadIdx.x] = s[threadIdx.x][0];
 }
 
-// P2M of charges q (and, when d3 is given, dipoles d3: 3 × N planar) into M (pitch per node)
 }  // namespace
 
 // ---------------------------------------------------------------- direct sums, FP64

@@ -146,7 +146,8 @@ int fmmb_batch_plan_instances(const fmmb_plan* plan, int64_t* ninst, int64_t* of
  * the given inputs (the plan's points, n of them, and its charges, or 3×n Stokeslets) — the M2L
  * block size (32, 64, 128 targets; when tune_blocks, re-cutting the plan's blocks, which its other
  * states share) — keeps the fastest and applies it, and records it for later plans of the same
- * method, kernel, order and N rounded down to a power of two. No result depends on it. The state's
+ * method, kernel, order and N rounded down to a power of two (one size for both precision paths: the
+ * fastest for the state tuned last). No result depends on it. The state's
  * expansions must be built again afterwards. out (may be NULL): 5 doubles, the block size, 0 and 4
  * (the FP64 M2L's chunk width and the near field's warps, which are no longer chosen), and the
  * chosen M2L and the near-field times in ms. */
@@ -177,7 +178,8 @@ int fmmb_matvec(fmmb_state* state, const double* xyz, const double* tau, int64_t
 int fmmb_matvec_dev(fmmb_state* state, const double* xyz_dev, const double* tau_dev, int64_t n, int outputs,
                     double* pot_dev, double* grad_dev);
 /* evaluate!(out, fmm, state, targets; output) (src/evaluate.jl:81-96): targets 3×nt, located
- * on the device (src/tree/locate.jl:10-22). */
+ * on the device (src/tree/locate.jl:10-22). How a target's near-field sum is split over lanes and warps
+ * depends on its leaf's sources and on how many of the targets share the leaf, and its last bits with it. */
 int fmmb_evaluate(fmmb_state* state, const double* targets, int64_t nt, int outputs, double* pot, double* grad);
 int fmmb_evaluate_dev(fmmb_state* state, const double* targets_dev, int64_t nt, int outputs, double* pot_dev, double* grad_dev);
 /* Waits for the state's work on the context's stream and reports what its kernels flagged:
