@@ -188,9 +188,10 @@ __device__ __forceinline__ void ki_fma2(uint64_t& d, uint64_t a, uint64_t b) {
 // Hadamard sums: a CTA keeps the 316 tables' block fb = blockIdx.x in shared memory, one CTA an SM; a warp per
 // sibling group, lane l the frequencies 2l, 2l + 1 of the block. The eight siblings' far
 // sources are the sourced children of their parent's colleagues, so each source's spectrum is read once
-// and multiplied into every sibling it is far from (seven of eight on average, in registers): what
-// bounds the sums is the L1 / shared-memory pipe, and a pair moves one table entry and an eighth of a
-// spectrum through it in place of one of each, with half the multiply-add instructions (f32x2).
+// and multiplied into every sibling it is far from (seven of eight on average, in registers): a pair moves one table
+// entry and an eighth of a spectrum through the L1 / shared-memory pipe in place of one of each, with half the
+// multiply-add instructions (f32x2). The pipe is 64 % busy; the table reads' latency and the multiply-adds' at four
+// warps a scheduler are the rest.
 // Each block's groups are handed out one by one to the warps of all its CTAs (next[fb]: they differ by a factor of
 // ten in far sources), and a colleague's spectra are loaded during the sums of the one before. Measured, the M2L
 // stage at 300,000 clustered points (3.63M pairs): p = 4 a warp per target 1.73 ms, sibling groups and no transforms

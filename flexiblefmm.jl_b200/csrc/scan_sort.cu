@@ -81,8 +81,8 @@ __global__ void k_tile_scan(const int* __restrict__ in, int64_t n, const int* __
 constexpr int RS_THREADS = 256;
 constexpr int RS_WARPS = RS_THREADS / 32;
 constexpr int RS_BINS = 256;
-// keys per thread: tiles of 4,096 keys, or of 1,024 where the larger ones would leave SMs idle (a tile's
-// scatter is a serial chain over its keys per thread)
+// keys per thread: tiles of 4,096 keys, or of 1,024 where the larger ones would leave some of the B200's 148 SMs
+// idle (a tile's scatter is a serial chain over its keys per thread)
 constexpr int RS_ITEMS_MAX = 16, RS_ITEMS_MIN = 4;
 constexpr int64_t RS_SMALL = 148ll * RS_THREADS * RS_ITEMS_MAX;
 
