@@ -23,7 +23,7 @@ using ld = long double;   // the blocks are formed in extended precision and rou
 
 // Wigner's d^l_{ab}(β), a ≥ |b|, for l = a..p at d[l], cb = cos β, ch and sh the cosine and sine of β/2:
 // d^a_{ab} = √C(2a, a + b) ch^(a+b) (−sh)^(a−b), then the three-term recurrence in the degree
-// (Varshalovich, Moskalev, Khersonskii, Quantum Theory of Angular Momentum, 1988, 4.8.1; upwards, as for the
+// (Varshalovich, Moskalev, Khersonskii, Quantum Theory of Angular Momentum, 1988, section 4.8; upwards, as for the
 // Jacobi polynomials, the stable direction)
 void wigner_d(int a, int b, int p, ld cb, ld ch, ld sh, ld* d) {
   ld v = 1;
